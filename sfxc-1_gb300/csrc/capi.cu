@@ -1116,9 +1116,10 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
       const float2 *twr = t.twrot.as<float2>();
       void *spec = c->spec.p;
       const int ww = plan_get(window_key(rot, count, nrows));
+      int *derr = c->derr.as<int>();
       q.kernel([=] {
         launch_window_fft(dchunk + N + first, count, 0, nrows, max_rows, win, twr, rot, nper, M, kpad, spec, tc_slots,
-                          tc_scale, st, ww);
+                          tc_scale, derr, st, ww);
       });
     }
     q.mark(sl.evs[ev + 3], st);
@@ -1314,7 +1315,7 @@ void prepare_outputs(sfxc_gpu_ctx *c, int k, IntegrationOut &out) {
   cudaStream_t st = c->st;
   float t_f1 = 0, t_f2 = 0, t_x = 0;
   CK(cudaStreamSynchronize(st));
-  if (*dev_err) throw Error(SFXC_GPU_ECUDA, "tensor-core X-step timed out waiting for its MMAs");
+  if (*dev_err) throw Error(SFXC_GPU_ECUDA, "a kernel timed out waiting for its copies or MMAs");
   // per chunk: F-step start and end, windowed FFT start (after the previous
   // X-step when that ran beside the F-step) and end, X-step end
   for (size_t q = 0; q + 5 <= ev; q += 5) {
@@ -1614,7 +1615,8 @@ int sfxc_gpu_autotune(sfxc_gpu_ctx *c, int32_t trials) {
       for (int v : {1, 2, 3, 4}) {
         const float ms = time_best([&] {
           launch_window_fft(t.dchunk + t.nstreams + first, count, 0, t.nrows, t.max_rows, rt.window.as<float>(),
-                            rt.twrot.as<float2>(), rot, nper, t.M, t.kpad, t.spec, t.tc_slots, t.tc_scale, c->st, v);
+                            rt.twrot.as<float2>(), rot, nper, t.M, t.kpad, t.spec, t.tc_slots, t.tc_scale,
+                            c->derr.as<int>(), c->st, v);
         });
         if (ms < best_t) {
           best_t = ms;
@@ -1688,7 +1690,7 @@ int sfxc_gpu_copy_spectra(sfxc_gpu_ctx *c, int32_t stream, float *out, size_t n)
     const int nper = c->p.window == WINDOW_NONE ? s.hop : s.rot;
     const sfxc_gpu_ctx::RotTables &t = c->rot_tables.at(s.rot);
     launch_window_fft(sd.as<StreamDev>(), 1, 0, (int)rows, (int)rows, t.window.as<float>(), t.twrot.as<float2>(),
-                      s.rot, nper, c->M, c->kpad, spec.p, 0, 1.0f, c->st);
+                      s.rot, nper, c->M, c->kpad, spec.p, 0, 1.0f, c->derr.as<int>(), c->st);
     CK(cudaGetLastError());
     CK(cudaMemcpy2DAsync(out, K * sizeof(float2), spec.p, c->kpad * sizeof(float2), K * sizeof(float2), rows,
                          cudaMemcpyDeviceToHost, c->st));
@@ -1776,7 +1778,7 @@ int sfxc_gpu_copy_spectra_noalloc(sfxc_gpu_ctx *c, int32_t stream, float *out, s
     const int nper = c->p.window == WINDOW_NONE ? s.hop : s.rot;
     const sfxc_gpu_ctx::RotTables &t = c->rot_tables.at(s.rot);
     launch_window_fft(dd, 1, 0, (int)rows, (int)rows, t.window.as<float>(), t.twrot.as<float2>(), s.rot, nper, c->M,
-                      c->kpad, spec, 0, 1.0f, c->st);
+                      c->kpad, spec, 0, 1.0f, c->derr.as<int>(), c->st);
     CK(cudaGetLastError());
     CK(cudaMemcpy2DAsync(out, K * sizeof(float2), spec, c->kpad * sizeof(float2), K * sizeof(float2), rows,
                          cudaMemcpyDeviceToHost, c->st));

@@ -7,8 +7,9 @@
 //                        (sfxc/src/delay_correction.cc:82-184) on the unpacked
 //                        samples of Bit2float_worker (sfxc/src/bit2float_worker.cc:327-425).
 //   window_fft_kernel    window, sideband flip, real FFT of 2M samples, channel
-//                        selection (delay_correction.cc:57-75); M/16 threads per row.
-// Both FFT stages are the register-resident radix-16 transforms of fft_reg.cuh.
+//                        selection (delay_correction.cc:57-75), for the longest transforms;
+//                        up to 4096 points in window_fft.cu.
+// These FFT stages are the register-resident radix-16 transforms of fft_reg.cuh.
 //   bitstat_kernel       per-code sample counts with cal-diode on/off split, from
 //                        popcounts (bit_statistics.cc:36-47, bit2float_worker.cc:341-346).
 //   xcorr_f32_kernel     X-step on CUDA cores, 4x4 stream tiles per thread
@@ -1181,7 +1182,7 @@ __global__ void __launch_bounds__(256) reduce_kernel(const float2 *__restrict__ 
 
 // ------------------------------------------------------------------------
 // launchers
-static int sm_count() {
+int sm_count() {
   static const int n = [] {  // initialised once, also when contexts are planned from several threads
     int dev = 0, v = 0;
     cudaGetDevice(&dev);
@@ -1304,11 +1305,6 @@ static void window_fft_launch(const StreamDev *d_streams, int nstreams, int row0
 
 #define SFXC_LOGN_SWITCH(logn, CALL) \
   switch (logn) {                    \
-    case 8: CALL(8); break;          \
-    case 9: CALL(9); break;          \
-    case 10: CALL(10); break;        \
-    case 11: CALL(11); break;        \
-    case 12: CALL(12); break;        \
     case 13: CALL(13); break;        \
     case 14: CALL(14); break;        \
     default: break; /* sizes outside 2^9..2^15 samples are rejected by set_parameters */ \
@@ -1316,7 +1312,10 @@ static void window_fft_launch(const StreamDev *d_streams, int nstreams, int row0
 
 void launch_window_fft(const StreamDev *d_streams, int nstreams, int row0, int nrows, int nrows_total,
                        const float *window, const float2 *tw_rot, int rot, int nper, int M, int kpad, void *spec,
-                       int tc_slots, float tc_scale, cudaStream_t st, int waves) {
+                       int tc_slots, float tc_scale, int *err, cudaStream_t st, int waves) {
+  if (launch_window_pack(d_streams, nstreams, row0, nrows, nrows_total, window, tw_rot, rot, nper, M, kpad, spec,
+                         tc_slots, tc_scale, err, st, waves))
+    return;
   const int logn = 30 - __builtin_clz((unsigned)rot);  // log2(rot / 2)
 #define SFXC_WIN(L)                                                                                            \
   (tc_slots == kTcSlots                                                                                         \
