@@ -820,14 +820,12 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
     d.sample_rate = ss.sample_rate;
     d.bandwidth = ss.bandwidth;
     d.oversamp = (int)std::round(ss.sample_rate / (2 * (double)ss.bandwidth));
-    d.frac_scale = -2.0 * M_PI / ss.sample_rate;
-    d.int_phase_q = M_PI / (2 * d.oversamp);
-    d.frac_scale_f = (float)d.frac_scale;
-    d.int_phase_q_f = (float)d.int_phase_q;
+    d.frac_scale_f = (float)(-2.0 / ss.sample_rate);
+    d.int_phase_q_f = (float)(1.0 / (2 * d.oversamp));
     d.half_bw_f = (float)(0.5 * ss.bandwidth);
     d.rate_per_bin_f = (float)((double)ss.sample_rate / kNd);
     d.sideband = ss.sideband == 'L' ? -1 : 1;
-    d.fringe_mult = -d.sideband * 2.0 * M_PI;
+    d.fringe_mult = -d.sideband * 2.0;
     d.center_freq = ss.channel_freq + d.sideband * ss.bandwidth * 0.5 + ss.lo_offset;
     d.lo_offset = ss.lo_offset;
     const double dt = time_diff(start, c->p.experiment_start_ticks);
@@ -1593,8 +1591,8 @@ int sfxc_gpu_autotune(sfxc_gpu_ctx *c, int32_t trials) {
     };
     int tuned = 0;
     {
-      const int cands[] = {4, 8, 12, 16, 24};
-      int best_v = 12;
+      const int cands[] = {2, 4, 6, 10, 16};
+      int best_v = 10;
       float best_t = 1e30f;
       for (int v : cands) {
         const float ms = time_best([&] { launch_fstep(t.dchunk, t.nstreams, t.max_blocks, c->tw256.as<float2>(), c->st, v); });

@@ -36,8 +36,8 @@ struct DevStatRange {
 // Per-block record of the F-step, written by block_params_kernel for the
 // blocks of one launch.
 struct BlockPar {
-  // phase-ramp start (rad, [0,2pi)), ramp step per bin, fringe phase at the
-  // block start, fringe phase step per sample
+  // in half turns (pi rad): phase-ramp start ([-1, 1]), ramp step per bin,
+  // fringe phase at the block start ([-1, 1]), fringe phase step per sample
   float4 ph;
   // cos and sin of 16 ramp steps, cos and sin of 16 fringe steps (the
   // per-thread recurrences of the block stage)
@@ -45,8 +45,8 @@ struct BlockPar {
   // bit of the block's first sample in the source when this block and the
   // next both lie inside one segment of recorded samples, else -1
   long long src_bit;
-  float amp;  // amplitude at the block centre
-  int32_t pad;
+  float amp;    // amplitude at the block centre
+  int32_t seg;  // plan segment of the block's first sample
 };
 static_assert(sizeof(BlockPar) == 48, "BlockPar layout");
 
@@ -77,12 +77,11 @@ struct StreamDev {
   int32_t sample_rate, bandwidth, oversamp, sideband;  // sideband +1 / -1
   double center_freq, lo_offset, start_phase;
   // per-stream quotients of Delay_correction::fractional_bit_shift, divided
-  // once here: -2 pi / sample_rate and pi / (2 oversamp); the ramp terms
-  // built from them end in FP32 and are computed there: -2 pi / sample_rate,
-  // pi / (2 oversamp), bandwidth / 2 and sample_rate / 256 as floats
-  double frac_scale, int_phase_q;
+  // once here, phases in half turns (pi rad); the ramp terms built from them
+  // end in FP32 and are computed there: -2 / sample_rate, 1 / (2 oversamp),
+  // bandwidth / 2 and sample_rate / 256
   float frac_scale_f, int_phase_q_f, half_bw_f, rate_per_bin_f;
-  // -sideband * 2 pi (the fringe phase's turn-to-radian factor)
+  // -sideband * 2 (the fringe phase's turns to half turns)
   double fringe_mult;
   // windowed FFT stage; slot: the stream's index in the job (its place in
   // the spectra layouts), also when the launch covers a subset of streams

@@ -43,6 +43,12 @@ __device__ __forceinline__ cpair mulw(cpair a, float x, float y) {
   return {fma2(a.re, wx, mul2(a.im, ny)), fma2(a.re, wy, mul2(a.im, wx))};
 }
 __device__ __forceinline__ cpair mulw(cpair a, float2 w) { return mulw(a, w.x, w.y); }
+// the same with the factor as (x, x, y, y): no register copies, one more product
+__device__ __forceinline__ cpair mulw(cpair a, float4 w) {
+  const float2 wx = make_float2(w.x, w.y), wy = make_float2(w.z, w.w);
+  const float2 n = mul2(a.im, dup2(-1.0f));
+  return {fma2(a.re, wx, mul2(n, wy)), fma2(a.re, wy, mul2(a.im, wx))};
+}
 
 // 4-point forward transform, outputs in natural order
 __device__ __forceinline__ void dft4(cpair &a0, cpair &a1, cpair &a2, cpair &a3) {
@@ -86,11 +92,10 @@ __device__ __forceinline__ void dft8(cpair *v) {
   v[7] = e3 - o3;
 }
 // 16-point forward transform as 4 x 4, natural order in and out.
-// HALF: the caller guarantees v[9..15] == 0 (the first stage drops the
+// half: the caller guarantees v[9..15] == 0 (the first stage drops the
 // additions of zeros).
-template <bool HALF = false>
-__device__ __forceinline__ void dft16(cpair (&v)[16]) {
-  if constexpr (HALF) {
+__device__ __forceinline__ void dft16(cpair (&v)[16], bool half = false) {
+  if (half) {
     {  // (v0, v4, v8, 0)
       const cpair a0 = v[0], a1 = v[4], a2 = v[8];
       const cpair t0 = a0 + a2, t1 = a0 - a2;

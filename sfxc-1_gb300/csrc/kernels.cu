@@ -1,11 +1,7 @@
 // CUDA kernels of the correlator-node path (sm_103a).
 //
-//   fstep_block_kernel   unpack (plan segments + 1/2-bit lookup) -> rfft(256)
-//                        -> fractional-delay phase ramp -> complex ifft(256)
-//                        -> fringe rotation; 16 threads per pair of blocks.
-//                        Delay_correction::fractional_bit_shift / fringe_stopping
-//                        (sfxc/src/delay_correction.cc:82-184) on the unpacked
-//                        samples of Bit2float_worker (sfxc/src/bit2float_worker.cc:327-425).
+//   block_params_kernel  per-block FP64 delay and fringe parameters of the F-step's
+//                        block stage (fstep.cu).
 //   window_fft_kernel    window, sideband flip, real FFT of 2M samples, channel
 //                        selection (delay_correction.cc:57-75), for the longest transforms;
 //                        up to 4096 points in window_fft.cu.
@@ -27,172 +23,6 @@
 namespace sfxc {
 
 // ------------------------------------------------------------------------
-// F-step, stage 1: 16 threads per pair of 256-sample blocks.  One forward
-// 256-point complex FFT of x_b + i x_{b+1} gives both real spectra
-// (X[k] +/- conj X[256-k]); per block: DC and Nyquist halved, phase ramp
-// exp(-i (c + k l)) on k <= 128, upper half zero, inverse 256-point FFT,
-// fringe rotation of the real part.  tw holds exp(-2 pi i m / 256), m < 256.
-//
-// Samples n of the pair's two blocks written as xs[n] and xs[256 + n] by this
-// half warp -> v[r] = (x_b[t + 16 r], x_b+1[t + 16 r]).  Only the half warp
-// synchronises (the other may be on another path).
-__device__ __forceinline__ void pair_from_scratch(float2 (&v)[16], const float *xs, int t) {
-  const unsigned half = (threadIdx.x & 16) ? 0xFFFF0000u : 0x0000FFFFu;
-  __syncwarp(half);
-#pragma unroll
-  for (int r = 0; r < 16; r++) v[r] = make_float2(xs[t + 16 * r], xs[kNd + t + 16 * r]);
-  __syncwarp(half);  // the FFT's first pass writes the scratch
-}
-
-// Pair (bl0, bl0 + 1) of a stream's blocks (indices from the stream's block0)
-// by the 16 threads t = 0..15 of a half warp, with a scratch of kFsScratch
-// float2; blocks at or past n_blocks give no output.  The
-// result goes through store(block, sample, value).  Both half warps of a warp
-// must call this together (warp barriers).
-constexpr int kFsScratch = kNd + kNd / 16 + 9 * 16;
-template <class Store>
-__device__ __forceinline__ void fstep_pair(const StreamDev &s, int bl0, int t, float2 *sm,
-                                           const float2 *__restrict__ tw, const float2 *ptab, Store store) {
-  const bool ok0 = bl0 < s.n_blocks, ok1 = bl0 + 1 < s.n_blocks;
-  float2 v[16];
-  {  // unpack the two blocks through the plan
-    const long long bit0 = ok0 ? s.bpar[bl0].src_bit : -1;
-    if (bit0 >= 0) {
-      // common case: both blocks inside one segment of recorded samples, so
-      // sample t + 16 r (r < 32 over the pair) sits at bit p + 16 r * bits of
-      // the stream; whole 32-bit words and funnel shifts, no segment walk
-      // (the input buffer has spare bytes after the last sample)
-      const uint32_t *w = reinterpret_cast<const uint32_t *>(s.src);
-      if (s.bits == 2) {
-        const int64_t p = bit0 + 2 * t;
-        const int64_t w0 = p >> 5;
-        const uint32_t sh = (uint32_t)p & 31;
-        uint32_t lo = __ldg(w + w0);
-#pragma unroll
-        for (int r = 0; r < 32; r++) {
-          const uint32_t hi = __ldg(w + w0 + r + 1);
-          const float x = code_value2(__funnelshift_r(lo, hi, sh) & 3);
-          if (r < 16)
-            v[r].x = x;
-          else
-            v[r - 16].y = x;
-          lo = hi;
-        }
-      } else {  // 1-bit: rolled loop through the scratch (small code for the instruction cache)
-        float *xs = reinterpret_cast<float *>(sm);
-#pragma unroll 1
-        for (int r = 0; r < 32; r++) {
-          const int64_t p = bit0 + t + 16 * r;
-          xs[t + 16 * r] = ((__ldg(w + (p >> 5)) >> (p & 31)) & 1) ? 5.0f : -5.0f;
-        }
-        pair_from_scratch(v, xs, t);
-      }
-    } else {  // segment boundaries inside the pair: rare per-sample walk, rolled, through the scratch
-      const int o0 = (s.block0 + bl0) * kNd;
-      int si = ok0 ? find_segment(s, o0) : 0;
-      float *xs = reinterpret_cast<float *>(sm);
-#pragma unroll 1
-      for (int r = 0; r < 32; r++) xs[t + 16 * r] = (r < 16 ? ok0 : ok1) ? gather_sample(s, o0 + t + 16 * r, si) : 0.0f;
-      pair_from_scratch(v, xs, t);
-    }
-  }
-  // The pair's forward transform and the two blocks' inverse ones share one
-  // code path (inverse as conj(FFT(conj Y))): h = 0 forward, h = 1, 2 the
-  // inverse of block h - 1.  Block 1's ramped half spectrum waits in the
-  // scratch behind the transform buffer, ext[16 r + t] for r < 9.
-  float2 *ext = sm + kNd + kNd / 16;
-  const float4 p0 = ok0 ? s.bpar[bl0].ph : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float4 p1 = ok1 ? s.bpar[bl0 + 1].ph : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 1
-  for (int h = 0; h < 3; h++) {
-    if (h == 2) {
-#pragma unroll
-      for (int r = 0; r < 9; r++) v[r] = ext[16 * r + t];
-#pragma unroll
-      for (int r = 9; r < 16; r++) v[r] = make_float2(0.f, 0.f);
-    }
-    // v[r] = X[t + 16 r]; the transform's reads of sm are complete on return
-    // (the inverse inputs are half spectra: v[9..15] == 0)
-    fft_reg<-1, 8, false, 15>(v, sm, t, tw, ptab, WarpSync(), h != 0);
-    if (h == 0) {
-      // split, halve DC/Nyquist, phase ramp; conj of block 0 into v, of block 1 into ext
-#pragma unroll
-      for (int r = 0; r < 16; r++) sm[padi(t + 16 * r)] = v[r];
-      __syncwarp();
-      float a_s, a_c, b_s, b_c;
-      sincosf(fmaf((float)t, p0.y, p0.x), &a_s, &a_c);
-      sincosf(fmaf((float)t, p1.y, p1.x), &b_s, &b_c);
-      const float4 st0 = ok0 ? s.bpar[bl0].steps : make_float4(1.f, 0.f, 1.f, 0.f);
-      const float4 st1 = ok1 ? s.bpar[bl0 + 1].steps : make_float4(1.f, 0.f, 1.f, 0.f);
-      const float as_c = st0.x, as_s = st0.y, bs_c = st1.x, bs_s = st1.y;
-#pragma unroll
-      for (int r = 0; r < 9; r++) {
-        const int k = t + 16 * r;
-        float2 f0 = make_float2(0.f, 0.f), f1 = make_float2(0.f, 0.f);
-        if (r < 8 || t == 0) {
-          const float2 xk = sm[padi(k & (kNd - 1))], xm = sm[padi((kNd - k) & (kNd - 1))];
-          const float hf = (k == 0 || k == kNd / 2) ? 0.25f : 0.5f;  // 1/2 of the split, DC and Nyquist halved again
-          const float er = hf * (xk.x + xm.x), ei = hf * (xk.y - xm.y);
-          const float orr = hf * (xk.y + xm.y), oi = -hf * (xk.x - xm.x);
-          // conj(F * (cos phi, -sin phi))
-          f0 = make_float2(er * a_c + ei * a_s, er * a_s - ei * a_c);
-          f1 = make_float2(orr * b_c + oi * b_s, orr * b_s - oi * b_c);
-        }
-        v[r] = f0;
-        ext[16 * r + t] = f1;
-        float c2 = a_c * as_c - a_s * as_s;
-        a_s = a_s * as_c + a_c * as_s;
-        a_c = c2;
-        c2 = b_c * bs_c - b_s * bs_s;
-        b_s = b_s * bs_c + b_c * bs_s;
-        b_c = c2;
-      }
-#pragma unroll
-      for (int r = 9; r < 16; r++) v[r] = make_float2(0.f, 0.f);
-      __syncwarp();  // the split's reads of sm before the next transform writes it
-    } else {
-      // v = conj(z), z the block's inverse transform: fringe rotation Re(z e^{-i phi}) x amplitude
-      const int bl = bl0 + h - 1;
-      if (bl < s.n_blocks) {
-        const float4 prm = h == 2 ? p1 : p0;
-        const float amp = s.bpar[bl].amp;
-        const float4 st = s.bpar[bl].steps;
-        const float sc = st.z, ss = st.w;
-        float rs, rc;
-        sincosf(fmaf((float)t, prm.w, prm.z), &rs, &rc);
-        rs *= amp;
-        rc *= amp;
-#pragma unroll
-        for (int r = 0; r < 16; r++) {
-          store(bl, t + 16 * r, v[r].x * rc - v[r].y * rs);
-          const float c2 = rc * sc - rs * ss;
-          rs = rs * sc + rc * ss;
-          rc = c2;
-        }
-      }
-    }
-  }
-}
-
-// F-step stage 1 as its own kernel (fringe-stopped samples to s.ts): 16
-// pairs of blocks per CTA of 256 threads.
-__global__ void __launch_bounds__(256, 4) fstep_block_kernel(const StreamDev *__restrict__ streams,
-                                                         const float2 *__restrict__ tw) {
-  extern __shared__ __align__(16) float2 sbuf[];  // 16 x kFsScratch
-  __shared__ float2 ptab[15 * pass_table_len<8>()];
-  const int t = threadIdx.x & 15, grp = threadIdx.x >> 4, warp = threadIdx.x >> 5;
-  const StreamDev &s = streams[blockIdx.y];
-  float *ts = s.ts;
-  fill_pass_table<8, 15>(ptab, tw, threadIdx.x, blockDim.x);
-  __syncthreads();
-  // 32 blocks per CTA and round, rounds strided over the stream's blocks
-  for (int first = blockIdx.x * 32; first < s.n_blocks; first += gridDim.x * 32) {
-    if (first + warp * 4 >= s.n_blocks) break;  // whole warps only (warp barriers); later rounds lie further out
-    fstep_pair(s, first + grp * 2, t, sbuf + grp * kFsScratch, tw, ptab,
-               [ts](int bl, int n, float x) { ts[(int64_t)bl * kNd + n] = x; });
-  }
-}
-
 // Per-block FP64 parameters of the F-step, one thread per 256-sample block
 // (all lanes busy on the reduced-rate FP64 pipe).  Follows
 // Delay_correction::do_task / fractional_bit_shift / fringe_stopping
@@ -253,7 +83,7 @@ __device__ __forceinline__ void block_params_one(const StreamDev &s, int bl, int
   const float frac = (float)(dis - integer_delay);
   const float tmp1 = frac * s.frac_scale_f;
   const float tmp2 = (float)(integer_delay & (4 * s.oversamp - 1)) * s.int_phase_q_f;
-  const float cterm = tmp2 - tmp1 * s.half_bw_f;
+  const float cterm = tmp2 - tmp1 * s.half_bw_f;  // half turns, as all phases of the record
   const float lterm = tmp1 * s.rate_per_bin_f;
   // the fringe phase in FP64 (tens of millions of turns); a zero LO offset or
   // phase model adds exact zeros, skipped
@@ -270,19 +100,19 @@ __device__ __forceinline__ void block_params_one(const StreamDev &s, int bl, int
     phi = phi + phase_0 * kInv2Pi;
     phi_end = phi_end + phase_1 * kInv2Pi;
   }
-  const double floor_phi = floor(phi);
-  phi = s.fringe_mult * (phi - floor_phi);
-  phi_end = s.fringe_mult * (phi_end - floor_phi);
+  const double turns = rint(phi);
+  phi = s.fringe_mult * (phi - turns);
+  phi_end = s.fringe_mult * (phi_end - turns);
   BlockPar bp;
-  bp.ph = make_float4(cterm - 6.28318548f * floorf(cterm * 0.159154937f), lterm, (float)phi,
+  bp.ph = make_float4(cterm - 2.0f * rintf(0.5f * cterm), lterm, (float)phi,
                       (float)((phi_end - phi) * (1.0 / kNd)));
-  sincosf(16.0f * bp.ph.y, &bp.steps.y, &bp.steps.x);
-  sincosf(16.0f * bp.ph.w, &bp.steps.w, &bp.steps.z);
+  sincospif(16.0f * bp.ph.y, &bp.steps.y, &bp.steps.x);
+  sincospif(16.0f * bp.ph.w, &bp.steps.w, &bp.steps.z);
   bp.amp = (float)ampl;
-  bp.pad = 0;
   // unpack source of the pair (bl, bl + 1) when both lie in one recorded segment
   const int o0 = (s.block0 + bl) * kNd;
-  const DevSegment sg = s.segs[find_segment(s, o0)];
+  bp.seg = find_segment(s, o0);
+  const DevSegment sg = s.segs[bp.seg];
   bp.src_bit = (bl + 1 < s.n_blocks && sg.src_bit >= 0 && o0 >= sg.out0 && o0 + 2 * kNd <= sg.out0 + sg.n)
                    ? sg.src_bit + (long long)(o0 - sg.out0) * s.bits
                    : -1;
@@ -1202,19 +1032,6 @@ void launch_fstep_block(const StreamDev *d_streams, int nstreams, int max_blocks
                         cudaStream_t st) {
   launch_block_params(d_streams, nstreams, max_blocks, st);
   launch_fstep(d_streams, nstreams, max_blocks, tw256, st, 0);
-}
-
-void launch_fstep(const StreamDev *d_streams, int nstreams, int max_blocks, const float2 *tw256, cudaStream_t st,
-                  int ctas_per_sm) {
-  // by default about three waves of 4 resident CTAs per SM, each CTA looping
-  // over rounds (measured against 1, 2, 4 and 6 waves on the 32-stream,
-  // 4096-channel job: 2 % faster than two, the others slower still); the
-  // autotuner may pick another count per shape
-  const int per_stream = std::max(1, (ctas_per_sm > 0 ? ctas_per_sm : 12) * sm_count() / nstreams);
-  dim3 grid(std::min((max_blocks + 31) / 32, per_stream), nstreams);
-  constexpr int smem = 16 * kFsScratch * sizeof(float2);
-  cudaFuncSetAttribute(fstep_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  fstep_block_kernel<<<grid, 256, smem, st>>>(d_streams, tw256);
 }
 
 void launch_unpack(const StreamDev *d_streams, int nstreams, int max_blocks, float *out, cudaStream_t st) {

@@ -15,7 +15,7 @@ void launch_fstep_block(const StreamDev *d_streams, int nstreams, int max_blocks
 // ctas_per_sm > 0: at most that many CTAs per SM in all (each striding over its stream's blocks)
 void launch_block_params(const StreamDev *d_streams, int nstreams, int max_blocks, cudaStream_t st,
                          int ctas_per_sm = 0);
-// ctas_per_sm: grid of the block stage, CTAs per SM over all streams (0: the default, 12)
+// ctas_per_sm: grid of the block stage, CTAs per SM over all streams (0: the default, 10)
 void launch_fstep(const StreamDev *d_streams, int nstreams, int max_blocks, const float2 *tw256, cudaStream_t st,
                   int ctas_per_sm = 0);
 void launch_unpack(const StreamDev *d_streams, int nstreams, int max_blocks, float *out, cudaStream_t st);
