@@ -227,7 +227,8 @@ struct Slot {
 
 // Host-side per-launch tables uploaded once per job.
 struct JobTables {
-  std::vector<int> blmap, tiles, blpairs;
+  std::vector<int> blmap, tiles, blpairs, blpart;
+  std::vector<int2> units;  // 8x8 tiles of the unbinned FP32 X-step
   int npad = 0, ntiles = 0;
 };
 
@@ -281,7 +282,7 @@ struct sfxc_gpu_ctx {
   std::vector<float> pc_weights;
   DevBuf pcacc, uvp;
   // device
-  DevBuf streamdev, tw256, ts, spec, acc, out, norms, flagfac, blmap, tiles, blpairs, items, bins,
+  DevBuf streamdev, tw256, ts, spec, acc, out, norms, flagfac, blmap, tiles, blpairs, blpart, units, items, bins,
       offsets, derr;
   DevBuf rowlist, segs;  // pulsar binning on the tensor cores: rows of each channel sorted by bin, and the runs
   DevBuf xpart;          // FP32 X-step: partial sums of its row blocks
@@ -620,6 +621,9 @@ void set_parameters(sfxc_gpu_ctx *c, const sfxc_correlation_params *p) {
     throw Error(SFXC_GPU_EINVAL, "the tensor-core X-step takes at most 64 streams per job");
   upload(c->blmap, jt.blmap.data(), jt.blmap.size() * 4, c->st);
   upload(c->tiles, jt.tiles.data(), jt.tiles.size() * 4, c->st);
+  jt.units = tile8_units(jt.blmap, jt.npad, N, jt.blpart, (int)c->bl.size());
+  upload(c->units, jt.units.data(), jt.units.size() * sizeof(int2), c->st);
+  upload(c->blpart, jt.blpart.data(), jt.blpart.size() * 4, c->st);
   upload(c->blpairs, jt.blpairs.data(), jt.blpairs.size() * 4, c->st);
   // twiddle tables: 256/128 for the block stage, rot and rot/2 for the windowed FFT
   std::vector<float2> tw;
@@ -931,7 +935,9 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
   c->derr.ensure(sizeof(int));
   q.memset(c->derr.p, 0, sizeof(int), st);
   if (!tc_x && !pulsar && !c->phased)
-    c->xpart.ensure(std::max<size_t>(16, xcorr_f32_scratch_bytes(c->jt.ntiles, c->jt.npad, K, max_rows, nbl, kpad)));
+    for (auto &r : ranges)
+      c->xpart.ensure(std::max<size_t>(
+          16, xcorr_f32_scratch_bytes((int)c->jt.units.size(), N, K, r.second - r.first, nbl, kpad)));
   // two sets of per-block records: chunk ch uses set ch & 1, so the next
   // chunk's are computed while the current chunk is still transformed
   for (int i = 0; i < N; i++) {
@@ -1155,8 +1161,8 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
           launches += 1;
         } else {
           q.kernel([=] {
-            launch_xcorr_f32(static_cast<float2 *>(specp), max_rows, kpad, N, npad, 0, nrows, K, tiles, ntiles, blmap,
-                             nbl, bins, nrows, acc, nullptr, 0, xs);
+            launch_xcorr_f32_binned(static_cast<float2 *>(specp), max_rows, kpad, N, npad, nrows, K, tiles, ntiles, blmap,
+                                    nbl, bins, acc, xs);
           });
         }
       } else if (tc_tma) {
@@ -1172,9 +1178,11 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
       } else {
         float2 *xpart = c->xpart.as<float2>();
         const size_t xcap = c->xpart.cap;
+        const int2 *units = c->units.as<int2>();
+        const int nunits = (int)c->jt.units.size(), *blpart = c->blpart.as<int>();
         q.kernel([=] {
-          launch_xcorr_f32(static_cast<float2 *>(specp), max_rows, kpad, N, npad, 0, nrows, K, tiles, ntiles, blmap, nbl,
-                           nullptr, 0, acc, xpart, xcap, xs);
+          launch_xcorr_f32(static_cast<float2 *>(specp), max_rows, kpad, N, npad, nrows, K, units, nunits, blmap, blpart,
+                           nbl, acc, xpart, xcap, xs);
         });
       }
       if (c->npc > 1) {  // the sub-integration into every phase centre

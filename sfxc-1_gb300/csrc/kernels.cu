@@ -8,10 +8,8 @@
 // These FFT stages are the register-resident radix-16 transforms of fft_reg.cuh.
 //   bitstat_kernel       per-code sample counts with cal-diode on/off split, from
 //                        popcounts (bit_statistics.cc:36-47, bit2float_worker.cc:341-346).
-//   xcorr_f32_kernel     X-step on CUDA cores, 4x4 stream tiles per thread
-//                        (Correlation_core::integration_step, correlation_core.cc:241-273).
-//   pulsar_bins_kernel / xcorr_f32_pulsar  bin per (FFT, channel) in FP64 and binned
-//                        accumulation (correlation_core_pulsar.cc:210-238).
+//   pulsar_bins_kernel / xcorr_f32_kernel  bin per (FFT, channel) in FP64 and binned
+//                        accumulation on CUDA cores (correlation_core_pulsar.cc:210-238).
 //   norm_* kernels       Correlation_core::integration_normalize (275-314).
 #include <algorithm>
 #include <cstdio>
@@ -641,36 +639,34 @@ __global__ void __launch_bounds__(256) bitstat_kernel(const StreamDev *__restric
 }
 
 // ------------------------------------------------------------------------
-// X-step on CUDA cores (Correlation_core::integration_step,
-// sfxc/src/correlation_core.cc:241-273; binned: Correlation_core_pulsar::
-// integration_step, sfxc/src/correlation_core_pulsar.cc:101-146).
-// spec: [stream][row][kpad] complex64.  Work items -- (32-channel tile, block
-// of rows, part of the stream-pair tiles) -- are dealt to persistent CTAs.  A
+// X-step on CUDA cores with pulsar binning (Correlation_core_pulsar::
+// integration_step, sfxc/src/correlation_core_pulsar.cc:101-146; without
+// bins: xcorr_f32.cu).
+// spec: [stream][row][kpad] complex64.  Work items -- (32-channel tile, part
+// of the stream-pair tiles) -- are dealt to persistent CTAs.  A
 // CTA stages R rows x npad streams x 32 channels per step through a 4-deep
 // cp.async ring (one barrier per R rows), so the loads of three steps are in
 // flight while one is multiplied; each thread owns one channel and up to TPW
 // tiles of 4x4 stream pairs (i in tile row I, j in tile column J, I <= J) in
-// registers, and adds them to the accumulators with float2 atomics when its
-// item ends, or, binned, when its channel's pulsar bin changes (acc[bin]).
+// registers, and adds them to acc[bin] with float2 atomics when its channel's
+// pulsar bin changes and when its item ends.
 // blmap[i*npad+j] gives (baseline << 1 | conj) or -1.
 __device__ __forceinline__ uint32_t smem_addr(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-template <int TPW, bool BINNED>
+template <int TPW>
 __global__ void __launch_bounds__(384, 1) xcorr_f32_kernel(const __grid_constant__ F32Args a) {
   extern __shared__ __align__(16) float2 xs[];  // kF32Stages x [R rows][npad streams][32 channels]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int nct = (a.K + 31) / 32;
-  const int nrows = a.r1 - a.r0;
-  const int nrb = (nrows + a.rblock - 1) / a.rblock;
-  const int nitems = nct * nrb * a.nparts;
+  const int nitems = nct * a.nparts;
   const int stage_f2 = a.R * a.npad * 32;  // float2 per stage
   const int chunks = a.R * a.npad * 16;    // 16-byte copies per stage
   for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
-    const int part = item % a.nparts, rb = (item / a.nparts) % nrb, ct = item / (a.nparts * nrb);
+    const int part = item % a.nparts, ct = item / a.nparts;
     const int k = ct * 32 + lane;
-    const int ra = a.r0 + rb * a.rblock, rz = min(a.r1, ra + a.rblock);
+    const int rz = a.nrows;
     const int t_end = min(a.ntiles, (part + 1) * a.tiles_per_part);
     int ti[TPW], tj[TPW];
     float2 v[TPW][4][4];
@@ -684,10 +680,9 @@ __global__ void __launch_bounds__(384, 1) xcorr_f32_kernel(const __grid_constant
 #pragma unroll
         for (int q = 0; q < 4; q++) v[t][p][q] = make_float2(0.f, 0.f);
     }
-    // add the register tiles to acc[bin] (bin 0 when not binned), or store
-    // them as this row block's partial sums (a.part), and clear them.  Each
-    // (bin, baseline, channel) entry has one writer thread per launch (or per
-    // row block with partial sums), so the results do not depend on timing.
+    // add the register tiles to acc[bin] and clear them.  Each (bin, baseline,
+    // channel) entry has one writer thread per launch, so the results do not
+    // depend on timing.
     auto flush = [&](int bin) {
       if (k >= a.K || bin < 0) return;
 #pragma unroll
@@ -701,24 +696,20 @@ __global__ void __launch_bounds__(384, 1) xcorr_f32_kernel(const __grid_constant
             if (m >= 0) {
               const float2 x = v[t][p][q];
               const float2 y = make_float2(x.x, (m & 1) ? -x.y : x.y);
-              if (a.part) {
-                a.part[((int64_t)rb * a.nbl + (m >> 1)) * a.kpad + k] = y;
-              } else {
-                // the entry's only writer in this launch: its adds land in
-                // program order, so the sum does not depend on timing; the
-                // atomic lets the thread go on without waiting for the load
-                atomicAdd(a.acc + ((int64_t)bin * a.nbl + (m >> 1)) * a.kpad + k, y);
-              }
+              // the entry's only writer in this launch: its adds land in
+              // program order, so the sum does not depend on timing; the
+              // atomic lets the thread go on without waiting for the load
+              atomicAdd(a.acc + ((int64_t)bin * a.nbl + (m >> 1)) * a.kpad + k, y);
             }
             v[t][p][q] = make_float2(0.f, 0.f);
           }
       }
     };
-    const int nsteps = (rz - ra + a.R - 1) / a.R;
+    const int nsteps = (rz + a.R - 1) / a.R;
     auto issue = [&](int step) {
       if (step < nsteps) {
         float2 *dst = xs + (step % kF32Stages) * stage_f2;
-        const int rs = ra + step * a.R;
+        const int rs = step * a.R;
         for (int c = threadIdx.x; c < chunks; c += blockDim.x) {
           const int rr = c / (a.npad * 16), rem = c - rr * (a.npad * 16), st = rem >> 4, cc = (rem & 15) * 2;
           const int row = rs + rr, kk = ct * 32 + cc;
@@ -743,14 +734,12 @@ __global__ void __launch_bounds__(384, 1) xcorr_f32_kernel(const __grid_constant
       const float2 *xst = xs + (step % kF32Stages) * stage_f2;
 #pragma unroll 1
       for (int rr = 0; rr < a.R; rr++) {
-        const int row = ra + step * a.R + rr;
+        const int row = step * a.R + rr;
         if (row >= rz) break;
-        if constexpr (BINNED) {
-          const int bin = k < a.K ? __ldg(a.bins + (int64_t)k * a.bins_rows + (row - a.r0)) : -1;
-          if (bin != cur) {
-            flush(cur);
-            cur = bin;
-          }
+        const int bin = k < a.K ? __ldg(a.bins + (int64_t)k * a.nrows + row) : -1;
+        if (bin != cur) {
+          flush(cur);
+          cur = bin;
         }
         const float2 *xr = xst + rr * a.npad * 32 + lane;
 #pragma unroll
@@ -774,22 +763,9 @@ __global__ void __launch_bounds__(384, 1) xcorr_f32_kernel(const __grid_constant
       }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    flush(BINNED ? cur : 0);
+    flush(cur);
     __syncthreads();  // the ring is refilled by the next item
   }
-}
-
-// Partial sums of the row blocks into the accumulators, in row-block order.
-__global__ void f32_part_reduce_kernel(const float2 *__restrict__ part, int nrb, int nbl, int kpad, int K,
-                                       float2 *__restrict__ acc) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
-  if (k >= K) return;
-  float2 s = acc[(int64_t)b * kpad + k];
-  for (int r = 0; r < nrb; r++) {
-    const float2 x = part[((int64_t)r * nbl + b) * kpad + k];
-    s = make_float2(s.x + x.x, s.y + x.y);
-  }
-  acc[(int64_t)b * kpad + k] = s;
 }
 
 // ------------------------------------------------------------------------
@@ -1172,7 +1148,7 @@ cudaError_t launch_reduce(const float2 *in, int nspec, int M, int nch, const flo
   return cudaGetLastError();
 }
 
-// Work split of the FP32 X-step for ntiles stream-pair tiles: parts of at
+// Work split of the binned FP32 X-step for ntiles stream-pair tiles: parts of at
 // most 36 tiles (12 warps x 3), the smallest tiles-per-warp that fits a part
 // into 12 warps, rows per step so that a step stages at most 32 KB.
 F32Plan xcorr_f32_plan(int ntiles, int npad) {
@@ -1189,84 +1165,37 @@ F32Plan xcorr_f32_plan(int ntiles, int npad) {
 }
 
 template <int TPW>
-static void f32_launch(const F32Args &a, const F32Plan &p, bool binned, cudaStream_t st) {
-  auto kern = binned ? xcorr_f32_kernel<TPW, true> : xcorr_f32_kernel<TPW, false>;
+static void f32_launch(const F32Args &a, const F32Plan &p, cudaStream_t st) {
+  auto kern = xcorr_f32_kernel<TPW>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
-  const int nct = (a.K + 31) / 32, nrows = a.r1 - a.r0;
-  const int nrb = (nrows + a.rblock - 1) / a.rblock;
-  const int nitems = nct * nrb * a.nparts;
-  kern<<<std::min(nitems, sm_count()), p.warps * 32, p.smem, st>>>(a);
+  kern<<<std::min((a.K + 31) / 32 * a.nparts, sm_count()), p.warps * 32, p.smem, st>>>(a);
 }
 
-// Row blocks of the unbinned FP32 X-step: about four work items per SM keep
-// the CTAs balanced; each block's partial sums go to scratch and are added in
-// block order.  Binned (pulsar) launches keep all rows in one block.
-static int f32_row_blocks(const F32Plan &p, int K, int nrows) {
-  const int nct = (K + 31) / 32;
-  return std::max(1, std::min((nrows + p.R - 1) / p.R, (4 * sm_count() + nct * p.nparts - 1) / (nct * p.nparts)));
-}
-
-size_t xcorr_f32_scratch_bytes(int ntiles, int npad, int K, int nrows, int nbl, int kpad) {
-  const F32Plan p = xcorr_f32_plan(ntiles, npad);
-  if (p.tpw <= 0 || nrows <= 0) return 0;
-  const int nrb = f32_row_blocks(p, K, nrows);
-  return nrb > 1 ? (size_t)nrb * nbl * kpad * sizeof(float2) : 0;
-}
-
-void launch_xcorr_f32(const float2 *spec, int nrows_total, int kpad, int nstreams, int npad, int r0, int r1, int K,
-                      const int *tiles, int ntiles, const int *blmap, int nbl, const int16_t *bins, int bins_rows,
-                      float2 *acc, float2 *scratch, size_t scratch_bytes, cudaStream_t st) {
-  if (r1 <= r0 || K <= 0) return;
+void launch_xcorr_f32_binned(const float2 *spec, int nrows_total, int kpad, int nstreams, int npad, int nrows, int K,
+                             const int *tiles, int ntiles, const int *blmap, int nbl, const int16_t *bins, float2 *acc,
+                             cudaStream_t st) {
+  if (nrows <= 0 || K <= 0) return;
   F32Plan p = xcorr_f32_plan(ntiles, npad);
   if (p.tpw <= 0) return;
-  const bool binned = bins != nullptr;
-  if (binned) {
-    // binned launches keep every row of a channel in one work item (each
-    // accumulator entry has one writer); finer parts of the tile set give the
-    // SMs enough items (each part stages the rows again, mostly from L2)
-    const int nct = (K + 31) / 32;
-    const int np = std::min(ntiles, std::max(p.nparts, (2 * sm_count() + nct - 1) / nct));
-    if (np > p.nparts) {
-      p.nparts = np;
-      p.tiles_per_part = (ntiles + np - 1) / np;
-      for (p.tpw = 1; p.tpw < 3 && (p.tiles_per_part + p.tpw - 1) / p.tpw > 12; p.tpw++) {
-      }
-      p.warps = (p.tiles_per_part + p.tpw - 1) / p.tpw;
+  // every row of a channel in one work item (each accumulator entry has one
+  // writer); finer parts of the tile set give the SMs enough items (each part
+  // stages the rows again, mostly from L2)
+  const int nct = (K + 31) / 32;
+  const int np = std::min(ntiles, std::max(p.nparts, (2 * sm_count() + nct - 1) / nct));
+  if (np > p.nparts) {
+    p.nparts = np;
+    p.tiles_per_part = (ntiles + np - 1) / np;
+    for (p.tpw = 1; p.tpw < 3 && (p.tiles_per_part + p.tpw - 1) / p.tpw > 12; p.tpw++) {
     }
+    p.warps = (p.tiles_per_part + p.tpw - 1) / p.tpw;
   }
-  F32Args a;
-  a.spec = spec;
-  a.nrows_total = nrows_total;
-  a.kpad = kpad;
-  a.nstreams = nstreams;
-  a.npad = npad;
-  a.r0 = r0;
-  a.r1 = r1;
-  a.K = K;
-  a.tiles = tiles;
-  a.ntiles = ntiles;
-  a.tiles_per_part = p.tiles_per_part;
-  a.nparts = p.nparts;
-  a.R = p.R;
-  a.blmap = blmap;
-  a.nbl = nbl;
-  a.bins = bins;
-  a.bins_rows = bins_rows;
-  a.acc = acc;
-  a.part = nullptr;
-  const int nrows = r1 - r0;
-  int nrb = binned ? 1 : f32_row_blocks(p, K, nrows);
-  if (nrb > 1 && (!scratch || scratch_bytes < (size_t)nrb * nbl * kpad * sizeof(float2))) nrb = 1;
-  a.rblock = ((nrows + nrb - 1) / nrb + p.R - 1) / p.R * p.R;
-  nrb = (nrows + a.rblock - 1) / a.rblock;
-  if (nrb > 1) a.part = scratch;
+  const F32Args a{spec, nrows_total, kpad, nstreams, npad, nrows, K, tiles, ntiles, p.tiles_per_part, p.nparts, p.R,
+                  blmap, nbl, bins, acc};
   switch (p.tpw) {
-    case 1: f32_launch<1>(a, p, binned, st); break;
-    case 2: f32_launch<2>(a, p, binned, st); break;
-    default: f32_launch<3>(a, p, binned, st); break;
+    case 1: f32_launch<1>(a, p, st); break;
+    case 2: f32_launch<2>(a, p, st); break;
+    default: f32_launch<3>(a, p, st); break;
   }
-  if (nrb > 1)
-    f32_part_reduce_kernel<<<dim3((K + 255) / 256, nbl), 256, 0, st>>>(scratch, nrb, nbl, kpad, K, acc);
 }
 
 void launch_pulsar_bins(int nrows, int K, double start_phase, double rate_term, double fft_duration,

@@ -1,6 +1,7 @@
 // Launch wrappers of the correlator-node kernels (kernels.cu, xcorr_tc.cu).
 #pragma once
 #include <cstdint>
+#include <vector>
 #include <cuda_runtime.h>
 
 #include "device.cuh"
@@ -31,20 +32,39 @@ bool launch_window_pack(const StreamDev *d_streams, int nstreams, int row0, int 
                         int tc_slots, float tc_scale, int *err, cudaStream_t st, int waves);
 int sm_count();
 void launch_bitstat(const StreamDev *d_streams, const int4 *d_items, int nitems, cudaStream_t st);
-// FP32 X-step (xcorr_f32_kernel): launch arguments and work split
+// FP32 X-step without binning (xcorr_f32.cu)
+struct TileArgs {
+  const float2 *spec;  // [stream][row][kpad] complex64
+  int nrows_total, kpad, nstreams, np8, npad, nrows, K;
+  const int2 *units;   // (I, J): 8x8 tile of stream pairs; (I, -J - 2): diagonal tiles I and J (-1: I alone)
+  int nunits, units_per_part, nparts, groups, nct, nsteps, R;  // groups of warps share a step's R rows
+  const int *blmap;    // [i * npad + j], i <= j: baseline << 1 | conjugated, or -1
+  int nbl;
+  float2 *acc;         // [baseline][kpad]
+  float2 *part;        // non-NULL: partial sums [slot][baseline][kpad], added later in order
+};
+// the units of a job and the part of them each baseline's sums come from
+std::vector<int2> tile8_units(const std::vector<int> &blmap, int npad, int nstreams, std::vector<int> &blpart, int nbl);
+// Scratch it wants for its shares' partial sums (0: none); with less, each
+// CTA takes one whole column.
+size_t xcorr_f32_scratch_bytes(int nunits, int nstreams, int K, int nrows, int nbl, int kpad);
+// rows 0..nrows-1 of spec into acc.  Deterministic: every accumulator entry
+// has one writer, partial sums are added in a fixed order.
+void launch_xcorr_f32(const float2 *spec, int nrows_total, int kpad, int nstreams, int npad, int nrows, int K,
+                      const int2 *units, int nunits, const int *blmap, const int *blpart, int nbl, float2 *acc,
+                      float2 *scratch, size_t scratch_bytes, cudaStream_t st);
+// FP32 X-step with pulsar binning (xcorr_f32_kernel): launch arguments and work split
 constexpr int kF32Stages = 4;         // cp.async ring depth
 constexpr int kF32StageBytes = 32768;  // rows x streams x 32 channels staged per step, at most
 struct F32Args {
   const float2 *spec;  // [stream][row][kpad] complex64
-  int nrows_total, kpad, nstreams, npad, r0, r1, K;
+  int nrows_total, kpad, nstreams, npad, nrows, K;
   const int *tiles;    // (I, J) per 4x4 stream-pair tile
-  int ntiles, tiles_per_part, nparts, rblock, R;
+  int ntiles, tiles_per_part, nparts, R;
   const int *blmap;
   int nbl;
-  const int16_t *bins;  // binned (pulsar): [channel][row] with row stride bins_rows, row 0 = r0; else NULL
-  int bins_rows;
+  const int16_t *bins;  // [channel][row]
   float2 *acc;          // [bin][baseline][kpad]
-  float2 *part;         // non-NULL: each row block's partial sums [block][baseline][kpad], added later in order
 };
 struct F32Plan {
   int nparts = 0, tiles_per_part = 0, tpw = 0, warps = 0, R = 0;
@@ -52,15 +72,11 @@ struct F32Plan {
 };
 // tpw == 0: the streams do not fit (npad x 256 B over 128 KB of staging)
 F32Plan xcorr_f32_plan(int ntiles, int npad);
-// Scratch the unbinned FP32 X-step wants for its row blocks' partial sums
-// (0: one block); with less, it runs the rows as one block.
-size_t xcorr_f32_scratch_bytes(int ntiles, int npad, int K, int nrows, int nbl, int kpad);
-// rows [r0, r1) of spec into acc; bins != NULL: binned, acc[bins[k][r - r0]].
-// Deterministic: every accumulator entry has one writer, partial sums are
-// added in a fixed order.
-void launch_xcorr_f32(const float2 *spec, int nrows_total, int kpad, int nstreams, int npad, int r0, int r1, int K,
-                      const int *tiles, int ntiles, const int *blmap, int nbl, const int16_t *bins, int bins_rows,
-                      float2 *acc, float2 *scratch, size_t scratch_bytes, cudaStream_t st);
+// rows 0..nrows-1 of spec into acc[bins[k][r]].  Deterministic: every
+// accumulator entry has one writer.
+void launch_xcorr_f32_binned(const float2 *spec, int nrows_total, int kpad, int nstreams, int npad, int nrows, int K,
+                             const int *tiles, int ntiles, const int *blmap, int nbl, const int16_t *bins, float2 *acc,
+                             cudaStream_t st);
 // pulsar bin of every (row, channel), FP64 in the reference's order: bins[k * nrows + r]
 void launch_pulsar_bins(int nrows, int K, double start_phase, double rate_term, double fft_duration,
                         const double *offsets, double g0, double g1, int nbins, int16_t *bins, cudaStream_t st);

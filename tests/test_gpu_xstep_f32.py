@@ -1,0 +1,41 @@
+"""The unbinned FP32 X-step where its work split changes: stream counts around
+the 8-stream tiles (one unit with eight row groups, two with four, several
+units, several parts), rows fewer than a step and more than a run, a
+reference station (tiles without baselines), against the FP64 restatement.
+
+Tolerance (relative L2 over all visibilities): as the block stage and windowed
+FFT feeding it, FP32 rounding below 1e-6 (sums of at most 256 rows in
+registers, then of those sums); twice that is allowed."""
+import numpy as np
+import pytest
+
+from oracle import jobs
+from sfxc_gpu import correlator, lib, scenario
+
+
+def make_job(streams, rows, ref=-1, pols=1, seed=7):
+    rate, nchan = 32_000_000, 256
+    st = scenario.cubic_stations(streams // pols, seed=seed, max_delay=1e-4, max_rate=1e-6)
+    sc = scenario.Scenario(stations=st, pols=("R", "L")[:pols], sample_rate=rate, bandwidth=rate // 2, nchan=nchan,
+                           integration_us=rows * nchan * 1_000_000 // rate, n_integrations=1, lead_us=1000, seed=seed,
+                           block_bytes=2000, reference_station=ref)
+    return scenario.build_job_bulk(sc)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("streams,rows,ref,pols", [(1, 5, -1, 1), (2, 700, -1, 1), (7, 33, -1, 1), (8, 300, -1, 1),
+                                                   (9, 40, -1, 1), (16, 1100, -1, 2), (17, 64, -1, 1),
+                                                   (24, 90, 3, 2), (33, 600, -1, 1), (42, 50, 20, 2)])
+def test_fp32_xstep_shapes(streams, rows, ref, pols):
+    j = make_job(streams, rows, ref, pols)
+    jj = dict(j, protocols=[[bytes(p) for p in s] for s in j["protocols"]])
+    want = jobs.correlate(jj, impl="oracle", precision=64)["cor"]
+    node = correlator.CorrelatorNode(0, lib.X_FP32)
+    try:
+        got, _ = node.correlate(j)
+    finally:
+        node.close()
+    (h0, v0), (h1, v1) = (correlator.split_output(x, j["number_channels"]) for x in (got, want))
+    assert h0 == h1
+    a, b = np.array(v0).astype(np.complex128), np.array(v1).astype(np.complex128)
+    assert np.linalg.norm(a - b) < 2e-6 * np.linalg.norm(b)
