@@ -175,7 +175,10 @@ int sfxc_gpu_push_protocol(sfxc_gpu_ctx *ctx, int32_t stream, const uint8_t *byt
  * the correlator output slice (file index, timeslice/uvw/statistics headers,
  * baseline headers and visibilities, byte-identical layout to
  * Correlation_core::integration_write); kind 1: one tsys record per stream
- * (the packed message of Correlation_core::tsys_write).  Return 0 to go on. */
+ * (the packed message of Correlation_core::tsys_write).  The bytes of kind 0
+ * stay where they are until the context's next integration (or its end), so
+ * a sink may note their address and copy them after the call; those of kind 1
+ * are gone when the sink returns.  Return 0 to go on. */
 typedef int (*sfxc_output_sink)(void *user, int32_t kind, const void *data, size_t n);
 
 /* UVW coordinates for the timeslice headers of the next and later

@@ -195,11 +195,19 @@ struct Ops {
   }
 };
 
+// Sizes of one output (a pulsar bin, a phase centre): its bytes are the
+// headers, then per baseline an 8-byte header and the output channels.  The
+// device writes the channels where they belong; the host fills in the rest.
+struct OutputLayout {
+  size_t head = 0, rec = 0, per = 0;  // header bytes, bytes per baseline, bytes per output
+};
+
 // What finish_integration needs of an enqueued integration.
 struct Pending {
   std::vector<int64_t> n_invalid;  // per stream, of this integration's unpack plan
   ticks_t start = 0;
-  size_t nvis = 0, ev = 0;
+  size_t ev = 0;
+  OutputLayout lay;
   int nout = 0, nphs = 0, launches = 0;
   bool pulsar = false;
   std::vector<std::pair<int64_t, int64_t>> nfl;
@@ -283,7 +291,7 @@ struct sfxc_gpu_ctx {
   DevBuf pcacc, uvp;
   // device
   DevBuf streamdev, tw256, ts, spec, acc, out, norms, flagfac, blmap, tiles, blpairs, blpart, units, items, bins,
-      offsets, derr;
+      offsets;
   DevBuf rowlist, segs;  // pulsar binning on the tensor cores: rows of each channel sorted by bin, and the runs
   DevBuf xpart;          // FP32 X-step: partial sums of its row blocks
   int bins_rows = 0;     // rows of the last integration's bin table (pulsar)
@@ -306,9 +314,9 @@ struct sfxc_gpu_ctx {
     void *spec = nullptr;
     std::vector<std::array<int, 3>> groups;
   } tune;
-  // bit-statistics counters of all streams (8 per stream), and the pinned
-  // landing area of an integration's results: visibilities, counters, the
-  // X-step's error flag (one readback copy each)
+  // bit-statistics counters of all streams (8 per stream) and the kernels'
+  // error flag; the pinned landing area of an integration's results holds
+  // them, then the outputs in their file layout (two readback copies)
   DevBuf hist;
   std::vector<StreamDev> hsd;
   // buffers of destroyed recordings, for the next ones
@@ -391,6 +399,11 @@ template <class T>
 void put(std::vector<uint8_t> &o, const T &v) {
   const uint8_t *p = reinterpret_cast<const uint8_t *>(&v);
   o.insert(o.end(), p, p + sizeof(T));
+}
+template <class T>
+void put(uint8_t *&o, const T &v) {
+  std::memcpy(o, &v, sizeof(T));
+  o += sizeof(T);
 }
 
 // Lag window of the spectral reduction when the ctrl file gives none:
@@ -671,18 +684,35 @@ std::vector<std::pair<int, int>> subint_ranges(const sfxc_gpu_ctx *c) {
   return r;
 }
 
-// bls: the baselines written (the job's, or the phased core's one (0, 0)
-// entry per sub-integration, Correlation_core_phased::create_baselines).
-void serialize_integration(sfxc_gpu_ctx *c, const std::vector<Baseline> &bls, const float2 *vis, int32_t source_nr,
-                           int centre, const std::vector<std::pair<int64_t, int64_t>> &nfl, std::vector<uint8_t> &o) {
-  const int N = (int)c->streams.size();
-  const int nbl = (int)bls.size();
-  put(o, source_nr);
-  // stations in stream order, each with its first stream
+// Stations in stream order, each with its first stream.
+std::vector<std::pair<int, int>> output_stations(const sfxc_gpu_ctx *c) {
   std::vector<std::pair<int, int>> stations;
   std::set<int> seen;
-  for (int i = 0; i < N; i++)
+  for (int i = 0; i < (int)c->streams.size(); i++)
     if (seen.insert(c->streams[i].station_number).second) stations.push_back({c->streams[i].station_number, i});
+  return stations;
+}
+
+OutputLayout output_layout(const sfxc_gpu_ctx *c, size_t nbl) {
+  OutputLayout l;
+  l.head = 20 + output_stations(c).size() * 32 + c->streams.size() * 24;
+  l.rec = 8 + (size_t)c->Kout * sizeof(float2);
+  l.per = l.head + nbl * l.rec;
+  return l;
+}
+// first output byte in the buffers: the headers are 4 bytes more than a
+// multiple of 8, so the first output's channels then lie on 8-byte boundaries
+constexpr size_t kOutBase = 4;
+
+// The headers of one output at o, around the channels already there.
+// bls: the baselines written (the job's, or the phased core's one (0, 0)
+// entry per sub-integration, Correlation_core_phased::create_baselines).
+void write_headers(sfxc_gpu_ctx *c, const std::vector<Baseline> &bls, int32_t source_nr, int centre,
+                   const std::vector<std::pair<int64_t, int64_t>> &nfl, uint8_t *o) {
+  const int N = (int)c->streams.size();
+  const int nbl = (int)bls.size();
+  const std::vector<std::pair<int, int>> stations = output_stations(c);
+  put(o, source_nr);
   put(o, (int32_t)(c->p.integration_nr + c->current_integration));
   put(o, (int32_t)nbl);
   put(o, (int32_t)stations.size());
@@ -693,10 +723,10 @@ void serialize_integration(sfxc_gpu_ctx *c, const std::vector<Baseline> &bls, co
     for (int k = 0; k < 3; k++) put(o, c->uvw[((size_t)s.second * c->npc + centre) * 3 + k]);
   }
   for (int i = 0; i < N; i++) {
-    o.push_back((uint8_t)c->streams[i].station_number);
-    o.push_back((uint8_t)c->p.frequency_nr);
-    o.push_back((uint8_t)(c->p.sideband == 'L' ? 0 : 1));
-    o.push_back((uint8_t)(c->streams[i].polarisation == 'R' ? 0 : 1));
+    put(o, (uint8_t)c->streams[i].station_number);
+    put(o, (uint8_t)c->p.frequency_nr);
+    put(o, (uint8_t)(c->p.sideband == 'L' ? 0 : 1));
+    put(o, (uint8_t)(c->streams[i].polarisation == 'R' ? 0 : 1));
     int lv[5];
     c->sc[i].stats.levels(lv);
     int32_t l[5];
@@ -709,21 +739,31 @@ void serialize_integration(sfxc_gpu_ctx *c, const std::vector<Baseline> &bls, co
     for (int k = 0; k < 5; k++) put(o, l[k]);
   }
   const int64_t total = (int64_t)c->nffts * c->M;
-  const size_t K = (size_t)c->Kout;  // output channels + 1
-  for (int b = 0; b < nbl; b++) {
+  const size_t vis = (size_t)c->Kout * sizeof(float2);
+  std::vector<int> flagged(N);
+  for (int i = 0; i < N; i++) {
     int lv[5];
-    c->sc[bls[b].a].stats.levels(lv);
-    int64_t w = bls[b].a == bls[b].b ? total - lv[4] : total - lv[4] - nfl[b].first;
-    put(o, (int32_t)std::max<int64_t>(w, 0));
-    o.push_back((uint8_t)c->streams[bls[b].a].station_number);
-    o.push_back((uint8_t)c->streams[bls[b].b].station_number);
-    o.push_back((uint8_t)((c->streams[bls[b].a].polarisation == 'R' ? 0 : 1) |
-                          ((c->streams[bls[b].b].polarisation == 'R' ? 0 : 1) << 1) |
-                          ((c->p.sideband == 'U' ? 1 : 0) << 2) | ((c->p.frequency_nr & 31) << 3)));
-    o.push_back((uint8_t)' ');
-    const uint8_t *d = reinterpret_cast<const uint8_t *>(vis + (size_t)b * K);
-    o.insert(o.end(), d, d + K * sizeof(float2));
+    c->sc[i].stats.levels(lv);
+    flagged[i] = lv[4];
   }
+  for (int b = 0; b < nbl; b++) {
+    const int64_t f = flagged[bls[b].a];
+    int64_t w = bls[b].a == bls[b].b ? total - f : total - f - nfl[b].first;
+    put(o, (int32_t)std::max<int64_t>(w, 0));
+    put(o, (uint8_t)c->streams[bls[b].a].station_number);
+    put(o, (uint8_t)c->streams[bls[b].b].station_number);
+    put(o, (uint8_t)((c->streams[bls[b].a].polarisation == 'R' ? 0 : 1) |
+                     ((c->streams[bls[b].b].polarisation == 'R' ? 0 : 1) << 1) |
+                     ((c->p.sideband == 'U' ? 1 : 0) << 2) | ((c->p.frequency_nr & 31) << 3)));
+    put(o, (uint8_t)' ');
+    o += vis;
+  }
+}
+
+// The kernels' error flag: behind the bit-statistics counters, cleared and
+// read back with them.
+int *device_error(sfxc_gpu_ctx *c) {
+  return c->hist.p ? reinterpret_cast<int *>(c->hist.as<uint8_t>() + c->streams.size() * 64) : nullptr;
 }
 
 // Node interval (the device search's answer) of the first block start of a
@@ -769,8 +809,8 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
   cudaStream_t st = c->st;
   // ---- host planning per stream (Bit2float_worker state machine replica)
   c->hsd.assign(N, StreamDev{});
-  c->hist.ensure((size_t)N * 64);
-  q.memset(c->hist.p, 0, (size_t)N * 64, st);
+  c->hist.ensure((size_t)N * 64 + 16);
+  q.memset(c->hist.p, 0, (size_t)N * 64 + 16, st);
   std::vector<int4> items;
   for (int i = 0; i < N; i++) {
     StreamCtx &s = c->sc[i];
@@ -932,8 +972,6 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
   // FP32 spectra: [stream][row][kpad]; TC spectra: [row][kpad][S stream slots], 8 bytes each
   // the TMA-fed kernel reads rows in groups of 8 (rows past a chunk's end cleared before its X-step)
   c->spec.ensure((size_t)(tc_x ? tc_slots : N) * (tc_x ? (max_rows + 7) / 8 * 8 : max_rows) * kpad * sizeof(float2));
-  c->derr.ensure(sizeof(int));
-  q.memset(c->derr.p, 0, sizeof(int), st);
   if (!tc_x && !pulsar && !c->phased)
     for (auto &r : ranges)
       c->xpart.ensure(std::max<size_t>(
@@ -1120,7 +1158,7 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
       const float2 *twr = t.twrot.as<float2>();
       void *spec = c->spec.p;
       const int ww = plan_get(window_key(rot, count, nrows));
-      int *derr = c->derr.as<int>();
+      int *derr = device_error(c);
       q.kernel([=] {
         launch_window_fft(dchunk + N + first, count, 0, nrows, max_rows, win, twr, rot, nper, M, kpad, spec, tc_slots,
                           tc_scale, derr, st, ww);
@@ -1135,7 +1173,7 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
       float2 *acc = c->acc.as<float2>();
       void *specp = c->spec.p;
       const int *blmap = c->blmap.as<int>(), *tiles = c->tiles.as<int>();
-      int *derr = c->derr.as<int>();
+      int *derr = device_error(c);
       const float inv_s2 = 1.0f / (tc_scale * tc_scale);
       if (c->phased) {
         q.kernel([=] { launch_phased(static_cast<float2 *>(specp), max_rows, kpad, N, r0c, nrows, K, nsub, acc, xs); });
@@ -1234,56 +1272,59 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
   // ---- normalisation and statistics, once the last X-step is done
   q.wait(st, sl.deps[3 * R]);
   q.mark(sl.evs[ev], st);
-  c->norms.ensure((size_t)N * 8);
   // outputs: the pulsar bins, or the phase centres (each normalised on its
-  // own); the phased array writes its sub-integration sums as they are
+  // own); the phased array writes its sub-integration sums as they are.  The
+  // last step writes them in the file layout, so that the host only fills in
+  // headers and passes the landed bytes on.
   const int nout = pulsar ? c->nbins : c->npc;
+  c->norms.ensure((size_t)nout * N * 8);
   const float2 *accs = c->npc > 1 ? c->pcacc.as<float2>() : c->acc.as<float2>();
-  c->out.ensure((size_t)std::max(nout * nbl, nphs) * K * sizeof(float2));
-  float2 *outp = c->out.as<float2>();
+  const OutputLayout lay = output_layout(c, c->phased ? nphs : nbl);
+  const size_t out_bytes = lay.per * (c->phased ? 1 : nout);
+  c->out.ensure(kOutBase + out_bytes);
+  uint8_t *const outp = c->out.as<uint8_t>() + kOutBase;
   if (c->phased) {
     const void *accp = c->acc.p;
     q.op([=] {
-      return cudaMemcpy2DAsync(outp, K * sizeof(float2), accp, kpad * sizeof(float2), K * sizeof(float2), nphs,
+      return cudaMemcpy2DAsync(outp + lay.head + 8, lay.rec, accp, kpad * sizeof(float2), K * sizeof(float2), nphs,
                                cudaMemcpyDeviceToDevice, st);
     });
   } else {
     const int *blp = c->blpairs.as<int>();
     double *norms = c->norms.as<double>();
     const double *ff = c->flagfac.as<double>();
-    q.kernel([=] {
-      for (int bin = 0; bin < nout; bin++)
-        launch_normalize(accs + (size_t)bin * nbl * kpad, kpad, M, N, nbl, blp, norms, ff, outp + (size_t)bin * nbl * K,
-                         st);
-    });
-  }
-  const float2 *vsrc = outp;
-  if (c->nch < M) {
-    c->rout.ensure((size_t)nout * nbl * c->Kout * sizeof(float2));
-    const int nch = c->nch, rnorm = c->rnorm;
-    const float *rmask = c->rmask.as<float>(), *rlag = c->rlag.as<float>();
-    const float2 *rtw = c->rtw.as<float2>();
+    const bool reduce = c->nch < M;
+    if (reduce) c->rout.ensure((size_t)nout * nbl * K * sizeof(float2));  // normalised spectra, compact
     float2 *rout = c->rout.as<float2>();
-    q.op([=] { return launch_reduce(outp, nout * nbl, M, nch, rmask, rlag, rnorm, rtw, rout, st); });
-    vsrc = rout;
-    launches += 1;
-  }
-  const size_t nvis = c->phased ? (size_t)nphs * c->Kout : (size_t)nout * nbl * c->Kout;
-  uint8_t *res = static_cast<uint8_t *>(sl.results.ensure(nvis * sizeof(float2) + (size_t)N * 64 + 16));
-  {
-    const void *histp = c->hist.p, *derrp = c->derr.p;
-    q.op([=] { return cudaMemcpyAsync(res, vsrc, nvis * sizeof(float2), cudaMemcpyDeviceToHost, st); });
-    q.op([=] { return cudaMemcpyAsync(res + nvis * sizeof(float2), histp, (size_t)N * 64, cudaMemcpyDeviceToHost, st); });
-    q.op([=] {
-      return cudaMemcpyAsync(res + nvis * sizeof(float2) + (size_t)N * 64, derrp, sizeof(int), cudaMemcpyDeviceToHost,
-                             st);
+    q.kernel([=] {
+      if (reduce)
+        launch_normalize(accs, kpad, M, N, nbl, nout, blp, norms, ff, reinterpret_cast<uint8_t *>(rout),
+                         (size_t)nbl * K * sizeof(float2), K * sizeof(float2), st);
+      else
+        launch_normalize(accs, kpad, M, N, nbl, nout, blp, norms, ff, outp + lay.head + 8, lay.per, lay.rec, st);
     });
+    launches += 2;
+    if (reduce) {
+      const int nch = c->nch, rnorm = c->rnorm;
+      const float *rmask = c->rmask.as<float>(), *rlag = c->rlag.as<float>();
+      const float2 *rtw = c->rtw.as<float2>();
+      q.op([=] {
+        return launch_reduce(rout, nbl, nout, M, nch, rmask, rlag, rnorm, rtw, outp + lay.head + 8, lay.per, lay.rec, st);
+      });
+      launches += 1;
+    }
+  }
+  const size_t res_out = (size_t)N * 64 + 16 + kOutBase;
+  uint8_t *res = static_cast<uint8_t *>(sl.results.ensure(res_out + out_bytes));
+  {
+    const void *histp = c->hist.p;
+    q.op([=] { return cudaMemcpyAsync(res + res_out, outp, out_bytes, cudaMemcpyDeviceToHost, st); });
+    q.op([=] { return cudaMemcpyAsync(res, histp, (size_t)N * 64 + 16, cudaMemcpyDeviceToHost, st); });
   }
   q.mark(sl.evs[ev + 1], st);
-  launches += 2 * nout;
   Pending &pd = sl.pend;
   pd.start = start;
-  pd.nvis = nvis;
+  pd.lay = lay;
   pd.nout = nout;
   pd.nphs = nphs;
   pd.ev = ev;
@@ -1297,27 +1338,27 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
 
 // After the recorded work has run: device error flag, timings, statistics,
 // output bytes to the sink.
-// The host side of a finished integration: its output bytes and tsys
-// records, made before any of them goes to the sink.
+// The host side of a finished integration: its output bytes (in the slot's
+// landing area) and tsys records, made before any of them goes to the sink.
 struct IntegrationOut {
-  std::vector<uint8_t> cor;
+  const uint8_t *cor = nullptr;
+  size_t n = 0;
   std::vector<std::vector<uint8_t>> tsys;
 };
 
 void prepare_outputs(sfxc_gpu_ctx *c, int k, IntegrationOut &out) {
   Slot &sl = *c->slots[k];
   Pending &pd = sl.pend;
-  const int N = (int)c->streams.size(), nbl = (int)c->bl.size();
-  const size_t nvis = pd.nvis, ev = pd.ev;
+  const int N = (int)c->streams.size();
+  const size_t ev = pd.ev;
   const int nout = pd.nout, nphs = pd.nphs;
   const bool pulsar = pd.pulsar;
   const ticks_t start = pd.start;
   const int launches = pd.launches;
   const std::vector<std::pair<int64_t, int64_t>> &nfl = pd.nfl;
   uint8_t *res = pd.res;
-  const float2 *vis = reinterpret_cast<const float2 *>(res);
-  const unsigned long long *hist = reinterpret_cast<const unsigned long long *>(res + nvis * sizeof(float2));
-  const int *dev_err = reinterpret_cast<const int *>(res + nvis * sizeof(float2) + (size_t)N * 64);
+  const unsigned long long *hist = reinterpret_cast<const unsigned long long *>(res);
+  const int *dev_err = reinterpret_cast<const int *>(res + (size_t)N * 64);
   cudaStream_t st = c->st;
   float t_f1 = 0, t_f2 = 0, t_x = 0;
   CK(cudaStreamSynchronize(st));
@@ -1356,18 +1397,16 @@ void prepare_outputs(sfxc_gpu_ctx *c, int k, IntegrationOut &out) {
     bs.sample_rate = c->streams[i].sample_rate;
     bs.base_sample_rate = c->p.sample_rate;
   }
-  // ---- output bytes (integration_write per bin) and tsys records
-  std::vector<uint8_t> &o = out.cor;
-  {
-    const size_t per_out = 20 + (size_t)N * (32 + 24) + (size_t)std::max(nbl, nphs) * (8 + (size_t)c->Kout * 8);
-    o.reserve(per_out * (size_t)std::max(1, nout));
-  }
+  // ---- output headers (integration_write per bin) and tsys records
+  uint8_t *o = res + (size_t)N * 64 + 16 + kOutBase;
+  out.cor = o;
   if (c->phased) {
-    serialize_integration(c, std::vector<Baseline>(nphs, Baseline{0, 0}), vis, 0, 0, nfl, o);
+    write_headers(c, std::vector<Baseline>(nphs, Baseline{0, 0}), 0, 0, nfl, o);
+    out.n = pd.lay.per;
   } else {
-    for (int bin = 0; bin < nout; bin++)
-      serialize_integration(c, c->bl, vis + (size_t)bin * nbl * c->Kout, pulsar ? bin : c->pc_file[bin],
-                            pulsar ? 0 : bin, nfl, o);
+    for (int bin = 0; bin < nout; bin++, o += pd.lay.per)
+      write_headers(c, c->bl, pulsar ? bin : c->pc_file[bin], pulsar ? 0 : bin, nfl, o);
+    out.n = pd.lay.per * (size_t)nout;
   }
   for (int i = 0; i < N && !c->phased; i++) {  // the phased core writes no tsys records
     out.tsys.emplace_back();
@@ -1386,7 +1425,7 @@ void prepare_outputs(sfxc_gpu_ctx *c, int k, IntegrationOut &out) {
 
 void deliver_outputs(const IntegrationOut &o, sfxc_output_sink sink, void *user) {
   if (!sink) return;
-  if (sink(user, 0, o.cor.data(), o.cor.size()) != 0) throw Error(SFXC_GPU_EINVAL, "output sink refused the data");
+  if (sink(user, 0, o.cor, o.n) != 0) throw Error(SFXC_GPU_EINVAL, "output sink refused the data");
   for (const std::vector<uint8_t> &t : o.tsys)
     if (sink(user, 1, t.data(), t.size()) != 0) throw Error(SFXC_GPU_EINVAL, "output sink refused the data");
 }
@@ -1622,7 +1661,7 @@ int sfxc_gpu_autotune(sfxc_gpu_ctx *c, int32_t trials) {
         const float ms = time_best([&] {
           launch_window_fft(t.dchunk + t.nstreams + first, count, 0, t.nrows, t.max_rows, rt.window.as<float>(),
                             rt.twrot.as<float2>(), rot, nper, t.M, t.kpad, t.spec, t.tc_slots, t.tc_scale,
-                            c->derr.as<int>(), c->st, v);
+                            device_error(c), c->st, v);
         });
         if (ms < best_t) {
           best_t = ms;
@@ -1692,15 +1731,19 @@ int sfxc_gpu_copy_spectra(sfxc_gpu_ctx *c, int32_t stream, float *out, size_t n)
     d.ts = ts.as<float>();
     d.bpar = bp.as<BlockPar>();
     upload(sd, &d, sizeof(StreamDev), c->st);
+    int err = 0;
+    if (device_error(c)) CK(cudaMemsetAsync(device_error(c), 0, sizeof(int), c->st));
     launch_fstep_block(sd.as<StreamDev>(), 1, s.n_blocks, c->tw256.as<float2>(), c->st);
     const int nper = c->p.window == WINDOW_NONE ? s.hop : s.rot;
     const sfxc_gpu_ctx::RotTables &t = c->rot_tables.at(s.rot);
     launch_window_fft(sd.as<StreamDev>(), 1, 0, (int)rows, (int)rows, t.window.as<float>(), t.twrot.as<float2>(),
-                      s.rot, nper, c->M, c->kpad, spec.p, 0, 1.0f, c->derr.as<int>(), c->st);
+                      s.rot, nper, c->M, c->kpad, spec.p, 0, 1.0f, device_error(c), c->st);
     CK(cudaGetLastError());
     CK(cudaMemcpy2DAsync(out, K * sizeof(float2), spec.p, c->kpad * sizeof(float2), K * sizeof(float2), rows,
                          cudaMemcpyDeviceToHost, c->st));
+    if (device_error(c)) CK(cudaMemcpyAsync(&err, device_error(c), sizeof(int), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
+    if (err) throw Error(SFXC_GPU_ECUDA, "a kernel timed out waiting for its copies");
     return (int)(rows * K * 2);
   } catch (const Error &e) {
     return fail(c, e);
@@ -1780,15 +1823,19 @@ int sfxc_gpu_copy_spectra_noalloc(sfxc_gpu_ctx *c, int32_t stream, float *out, s
     // every scratch element read below is written first by the same call, so
     // nothing is cleared; the descriptor copy is ordered on the context stream
     CK(cudaMemcpyAsync(dd, &d, sizeof(StreamDev), cudaMemcpyHostToDevice, c->st));
+    int err = 0;
+    if (device_error(c)) CK(cudaMemsetAsync(device_error(c), 0, sizeof(int), c->st));
     launch_fstep_block(dd, 1, s.n_blocks, c->tw256.as<float2>(), c->st);
     const int nper = c->p.window == WINDOW_NONE ? s.hop : s.rot;
     const sfxc_gpu_ctx::RotTables &t = c->rot_tables.at(s.rot);
     launch_window_fft(dd, 1, 0, (int)rows, (int)rows, t.window.as<float>(), t.twrot.as<float2>(), s.rot, nper, c->M,
-                      c->kpad, spec, 0, 1.0f, c->derr.as<int>(), c->st);
+                      c->kpad, spec, 0, 1.0f, device_error(c), c->st);
     CK(cudaGetLastError());
     CK(cudaMemcpy2DAsync(out, K * sizeof(float2), spec, c->kpad * sizeof(float2), K * sizeof(float2), rows,
                          cudaMemcpyDeviceToHost, c->st));
+    if (device_error(c)) CK(cudaMemcpyAsync(&err, device_error(c), sizeof(int), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
+    if (err) throw Error(SFXC_GPU_ECUDA, "a kernel timed out waiting for its copies");
     return (int)(rows * K * 2);
   } catch (const Error &e) {
     return fail(c, e);

@@ -801,11 +801,13 @@ __global__ void pulsar_bins_kernel(int nrows, int K, double start_phase, double 
 
 // ------------------------------------------------------------------------
 // Normalisation.  norms[i] = max(1, sum_k Re acc[auto_i][k] / M) in FP64.
-__global__ void norm_autos_kernel(const float2 *__restrict__ acc, int kpad, int M, int nstreams, double *norms) {
+__global__ void norm_autos_kernel(const float2 *__restrict__ acc, int kpad, int M, int nstreams, int nbl,
+                                  double *norms) {
   __shared__ double red[256];
   const int i = blockIdx.x;
+  acc += ((int64_t)blockIdx.y * nbl + i) * kpad;
   double s = 0.0;
-  for (int k = threadIdx.x; k <= M; k += blockDim.x) s += (double)acc[(int64_t)i * kpad + k].x;
+  for (int k = threadIdx.x; k <= M; k += blockDim.x) s += (double)acc[k].x;
   red[threadIdx.x] = s;
   __syncthreads();
   for (int w = blockDim.x / 2; w > 0; w >>= 1) {
@@ -814,18 +816,24 @@ __global__ void norm_autos_kernel(const float2 *__restrict__ acc, int kpad, int 
   }
   if (threadIdx.x == 0) {
     double n = red[0] / M;
-    norms[i] = n < 1 ? 1 : n;
+    norms[blockIdx.y * nstreams + i] = n < 1 ? 1 : n;
   }
 }
 
-// out[b][k] (compact M+1) = normalised visibility; flagfac[b] = N1*N2 (crosses).
+// Output z (a pulsar bin or phase centre; accumulators and norms one after
+// another): M + 1 normalised channels of baseline b at out + z out_stride + b
+// bl_stride bytes, which may lie on 4-byte boundaries only (the output's
+// file layout), so the parts are stored singly; flagfac[b] = N1*N2 (crosses).
 // A cross baseline's FP64 norm is the same for all its channels: one thread
 // of the CTA (all of whose threads share the baseline) computes it.
 __global__ void normalize_kernel(const float2 *__restrict__ acc, int kpad, int M, int nstreams, int nbl,
                                  const int *__restrict__ bl, const double *__restrict__ norms,
-                                 const double *__restrict__ flagfac, float2 *__restrict__ out) {
+                                 const double *__restrict__ flagfac, uint8_t *__restrict__ out, size_t out_stride,
+                                 size_t bl_stride) {
   const int b = blockIdx.y;
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  acc += (int64_t)blockIdx.z * nbl * kpad;
+  norms += (int64_t)blockIdx.z * nstreams;
   __shared__ float cross_norm;
   if (b >= nstreams && threadIdx.x == 0)
     cross_norm = (float)sqrt(flagfac[b] * norms[bl[2 * b]] * norms[bl[2 * b + 1]]);
@@ -839,7 +847,9 @@ __global__ void normalize_kernel(const float2 *__restrict__ acc, int kpad, int M
     const float norm = cross_norm;
     o = make_float2(v.x / norm, v.y / norm);
   }
-  out[(int64_t)b * (M + 1) + k] = o;
+  float *d = reinterpret_cast<float *>(out + blockIdx.z * out_stride + b * bl_stride) + 2 * k;
+  d[0] = o.x;
+  d[1] = o.y;
 }
 
 // ------------------------------------------------------------------------
@@ -931,7 +941,8 @@ __device__ void smem_fft_radix2(float2 *a, int logn, int sign, const float2 *__r
 __global__ void __launch_bounds__(256) reduce_kernel(const float2 *__restrict__ in, int M, int logM, int nch,
                                                      int lognch, const float *__restrict__ mask,
                                                      const float *__restrict__ lagwin, int normalize,
-                                                     const float2 *__restrict__ tw2M, float2 *__restrict__ out) {
+                                                     const float2 *__restrict__ tw2M, int nbl,
+                                                     uint8_t *__restrict__ out, size_t out_stride, size_t bl_stride) {
   extern __shared__ __align__(16) float2 rsm[];
   float2 *a = rsm;                                   // M complex
   float *lag = reinterpret_cast<float *>(rsm + M);   // 2 nch lags
@@ -975,14 +986,16 @@ __global__ void __launch_bounds__(256) reduce_kernel(const float2 *__restrict__ 
   __syncthreads();
   smem_fft_radix2(a, lognch, -1, tw2M, M);
   // r2c split: A[k] = E + W^k O, W = exp(-2 pi i / 2nch) = tw2M[M / nch]
-  float2 *Y = out + (size_t)blockIdx.x * (nch + 1);
+  // spectrum blockIdx.x: baseline of an output, 4-byte aligned as normalize_kernel's
+  float *Y = reinterpret_cast<float *>(out + blockIdx.x / nbl * out_stride + blockIdx.x % nbl * bl_stride);
   const float scale = (float)(2 * M);
   for (int k = threadIdx.x; k <= nch; k += blockDim.x) {
     const float2 zk = a[k & (nch - 1)], zc = a[(nch - k) & (nch - 1)];
     const float er = 0.5f * (zk.x + zc.x), ei = 0.5f * (zk.y - zc.y);
     const float orr = 0.5f * (zk.y + zc.y), oi = -0.5f * (zk.x - zc.x);
     const float2 w = __ldg(tw2M + (size_t)k * (M / nch));
-    Y[k] = make_float2((er + (orr * w.x - oi * w.y)) / scale, (ei + (orr * w.y + oi * w.x)) / scale);
+    Y[2 * k] = (er + (orr * w.x - oi * w.y)) / scale;
+    Y[2 * k + 1] = (ei + (orr * w.y + oi * w.x)) / scale;
   }
 }
 
@@ -1137,14 +1150,17 @@ void launch_pc_dump(float2 *acc, float2 *pcacc, const UvShift *uvp, int nstreams
   if (nbl > 0) pc_dump_kernel<<<dim3((K + 255) / 256, nbl), 256, 0, st>>>(acc, pcacc, uvp, nstreams, nbl, kpad, K, npc);
 }
 
-cudaError_t launch_reduce(const float2 *in, int nspec, int M, int nch, const float *mask, const float *lag_window,
-                          int normalize, const float2 *tw2M, float2 *out, cudaStream_t st) {
+cudaError_t launch_reduce(const float2 *in, int nbl, int nout, int M, int nch, const float *mask,
+                          const float *lag_window, int normalize, const float2 *tw2M, uint8_t *out, size_t out_stride,
+                          size_t bl_stride, cudaStream_t st) {
+  const int nspec = nbl * nout;
   if (nspec <= 0) return cudaSuccess;
   const int logM = 31 - __builtin_clz((unsigned)M), lognch = 31 - __builtin_clz((unsigned)nch);
   const size_t smem = (size_t)M * sizeof(float2) + (size_t)2 * nch * sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(reduce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  reduce_kernel<<<nspec, 256, smem, st>>>(in, M, logM, nch, lognch, mask, lag_window, normalize, tw2M, out);
+  reduce_kernel<<<nspec, 256, smem, st>>>(in, M, logM, nch, lognch, mask, lag_window, normalize, tw2M, nbl, out,
+                                          out_stride, bl_stride);
   return cudaGetLastError();
 }
 
@@ -1204,11 +1220,11 @@ void launch_pulsar_bins(int nrows, int K, double start_phase, double rate_term, 
                                                                   offsets, g0, g1, nbins, bins);
 }
 
-void launch_normalize(const float2 *acc, int kpad, int M, int nstreams, int nbl, const int *bl, double *norms,
-                      const double *flagfac, float2 *out, cudaStream_t st) {
-  norm_autos_kernel<<<nstreams, 256, 0, st>>>(acc, kpad, M, nstreams, norms);
-  normalize_kernel<<<dim3((M + 1 + 255) / 256, nbl), 256, 0, st>>>(acc, kpad, M, nstreams, nbl, bl, norms, flagfac,
-                                                                    out);
+void launch_normalize(const float2 *acc, int kpad, int M, int nstreams, int nbl, int nout, const int *bl, double *norms,
+                      const double *flagfac, uint8_t *out, size_t out_stride, size_t bl_stride, cudaStream_t st) {
+  norm_autos_kernel<<<dim3(nstreams, nout), 256, 0, st>>>(acc, kpad, M, nstreams, nbl, norms);
+  normalize_kernel<<<dim3((M + 1 + 255) / 256, nbl, nout), 256, 0, st>>>(acc, kpad, M, nstreams, nbl, bl, norms,
+                                                                          flagfac, out, out_stride, bl_stride);
 }
 
 }  // namespace sfxc

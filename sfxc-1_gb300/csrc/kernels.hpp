@@ -96,8 +96,10 @@ cudaError_t launch_xcorr_tc(const void *spec, int nrows, int kpad, int K, const 
 cudaError_t launch_xcorr_tc_gather(const void *spec, int slots, int nrows, int kpad, int K, int nstreams,
                                    const int *blmap, int npad, int nbl, int nbins, const int *rowlist, int list_len,
                                    const int2 *segs, float inv_scale2, float2 *acc, int *err, cudaStream_t st);
-void launch_normalize(const float2 *acc, int kpad, int M, int nstreams, int nbl, const int *bl, double *norms,
-                      const double *flagfac, float2 *out, cudaStream_t st);
+// nout outputs of nbl baselines each, one after another in acc ([output][baseline][kpad]) and norms; the M + 1
+// channels of output z and baseline b go to out + z out_stride + b bl_stride (bytes, multiples of 4)
+void launch_normalize(const float2 *acc, int kpad, int M, int nstreams, int nbl, int nout, const int *bl, double *norms,
+                      const double *flagfac, uint8_t *out, size_t out_stride, size_t bl_stride, cudaStream_t st);
 // Sub-integration dump with extra phase centres: acc[b][k] (b < nbl, k < K,
 // rows kpad apart) added to every centre's accumulator pcacc[c][b][k], rotated
 // for c >= 1 on cross baselines (b >= nstreams) by uvp[(c - 1) nbl + b] =
@@ -109,11 +111,13 @@ void launch_pc_dump(float2 *acc, float2 *pcacc, const UvShift *uvp, int nstreams
 // nrows_total rows per stream slot, kpad apart).
 void launch_phased(const float2 *spec, int nrows_total, int kpad, int nstreams, int r0, int nrows, int K, int nsub,
                    float2 *acc, cudaStream_t st);
-// Spectral reduction of nspec normalised spectra of M + 1 channels to nch + 1
+// Spectral reduction of nout x nbl normalised spectra of M + 1 channels to nch + 1
 // channels (M, nch powers of two, nch < M); mask: M + 1 values, lag_window:
 // 2 nch values, tw2M: exp(-2 pi i k / 2M) for k < 2M.
-cudaError_t launch_reduce(const float2 *in, int nspec, int M, int nch, const float *mask, const float *lag_window,
-                          int normalize, const float2 *tw2M, float2 *out, cudaStream_t st);
+// placed as launch_normalize does
+cudaError_t launch_reduce(const float2 *in, int nbl, int nout, int M, int nch, const float *mask,
+                          const float *lag_window, int normalize, const float2 *tw2M, uint8_t *out, size_t out_stride,
+                          size_t bl_stride, cudaStream_t st);
 // Phase-cal folding: run k adds the samples of its bytes data[off, off + n)
 // to accumulator row `row` (pb * (8 / bits) int32 bins), byte j to byte-bin
 // (bin0 + j) mod pb.

@@ -26,6 +26,45 @@ def _bytes_ptr(b):
     return arr
 
 
+# Output bytes larger than this are copied by several threads: a fresh object
+# of that size is new pages, whose first touch costs more than the copy.
+_COPY_CHUNK = 4 << 20
+
+
+_NEW_BYTES = C.PYFUNCTYPE(C.py_object, C.c_char_p, C.c_ssize_t)(("PyBytes_FromStringAndSize", C.pythonapi))
+_NEW_BYTEARRAY = C.PYFUNCTYPE(C.py_object, C.c_char_p, C.c_ssize_t)(("PyByteArray_FromStringAndSize", C.pythonapi))
+_BYTES_AT = C.PYFUNCTYPE(C.c_void_p, C.py_object)(("PyBytes_AsString", C.pythonapi))
+_BYTEARRAY_AT = C.PYFUNCTYPE(C.c_void_p, C.py_object)(("PyByteArray_AsString", C.pythonapi))
+
+
+def _uninitialised(kind, n):
+    """A bytes or bytearray object of n bytes not yet written, and its address."""
+    obj = (_NEW_BYTES if kind is bytes else _NEW_BYTEARRAY)(None, n)
+    return obj, (_BYTES_AT if kind is bytes else _BYTEARRAY_AT)(obj)
+
+
+def _collect(pieces, kind):
+    """One object of the bytes at pieces [(address, n)], one after another.
+    The copies are foreign calls (ctypes.memmove), so other threads driving
+    other contexts keep the interpreter meanwhile."""
+    total = sum(n for _, n in pieces)
+    obj, dst = _uninitialised(kind, total)
+    chunks = []
+    for src, n in pieces:
+        step = n if n < 2 * _COPY_CHUNK else max(_COPY_CHUNK, -(-n // 8))
+        for o in range(0, n, step or 1):
+            chunks.append((dst + o, src + o, min(step, n - o)))
+        dst += n
+    if total < 2 * _COPY_CHUNK:
+        for c in chunks:
+            C.memmove(*c)
+    else:
+        with ThreadPoolExecutor(max_workers=min(8, len(chunks), -(-total // _COPY_CHUNK))) as pool:
+            for f in [pool.submit(C.memmove, *c) for c in chunks]:
+                f.result()
+    return obj
+
+
 def correlation_params(job):
     """The sfxc_correlation_params of a job dict (the keys of
     oracle/jobs.correlate: the same dicts drive the reference checker, the C
@@ -160,20 +199,23 @@ class CorrelatorNode:
 
     def run_integration(self):
         """Returns (output bytes (bytes or bytearray), [tsys record bytes per stream])."""
+        return self._run(bytearray)
+
+    def _run(self, kind):
         out, tsys = [], []
 
-        def sink(user, kind, data, n):
-            # the copy is a foreign call (ctypes.memmove), so other threads
-            # driving other contexts keep the interpreter meanwhile
-            b = bytearray(n)
-            if n:
-                C.memmove((C.c_char * n).from_buffer(b), data, n)
-            (out if kind == 0 else tsys).append(bytes(b) if kind else b)
+        def sink(user, what, data, n):
+            # the output bytes stay where they are until the context's next
+            # integration: copied below, after the call
+            if what == 0:
+                out.append((data or 0, n))
+            else:
+                tsys.append(C.string_at(data, n))
             return 0
 
         cb = L.SINK(sink)
         self._check(self._lib.sfxc_gpu_run_integration(self._h, cb, None))
-        return (out[0] if len(out) == 1 else b"".join(out)), tsys
+        return _collect(out, kind if len(out) == 1 else bytes), tsys
 
     def correlate(self, job):
         """Run every integration of a job dict; returns (cor bytes, tsys bytes)."""
@@ -184,10 +226,10 @@ class CorrelatorNode:
                 self.set_uvw(job["uvw"][it])
             for k in range(self.nstreams):
                 self.push_protocol(k, job["protocols"][k][it])
-            o, t = self.run_integration()
+            o, t = self._run(bytes)
             cor.append(o)
             tsys += t
-        return b"".join(cor), b"".join(tsys)
+        return b"".join(cor), b"".join(tsys)  # a single bytes object is returned as it is
 
     def unpacked(self, stream, n):
         out = np.empty(n, dtype=np.float32)
@@ -578,11 +620,11 @@ class Batch:
         outs = [([], []) for _ in self.nodes]
 
         def sink(user, kind, data, n):
-            b = bytearray(n)
-            if n:
-                C.memmove((C.c_char * n).from_buffer(b), data, n)
             o = outs[user or 0]
-            (o[0] if kind == 0 else o[1]).append(b)
+            if kind == 0:  # stays where it is until the context's next run
+                o[0].append((data or 0, n))
+            else:
+                o[1].append(C.string_at(data, n))
             return 0
 
         cb = L.SINK(sink)
@@ -594,8 +636,8 @@ class Batch:
             rc = self._lib.sfxc_gpu_batch_run_counts(self._h, cnt, cb, users)
         if rc < 0:
             raise L.SfxcError(rc, self._lib.sfxc_gpu_global_error().decode())
-        # one output buffer is passed on as it is (bytearray); several are joined
-        return [(o[0] if len(o) == 1 else b"".join(o), [bytes(x) for x in t]) for o, t in outs]
+        # one output is a bytearray, several are joined
+        return [(_collect(o, bytearray if len(o) == 1 else bytes), t) for o, t in outs]
 
     def last_ms(self):
         return float(self._lib.sfxc_gpu_batch_last_ms(self._h))
