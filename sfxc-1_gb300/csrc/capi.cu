@@ -1123,6 +1123,29 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
     q.kernel([=] { launch_bitstat(sdev, ditems, nitems, st); });
   }
   int launches = items.empty() ? 0 : 1;
+  // Pulsar binning: the bin of every (row, channel) of the integration (its
+  // one chunk) and the sort by bin need no spectra, so they run on the third
+  // stream beside the F-step.
+  if (pulsar) {
+    const int nrows = ranges[0].second - ranges[0].first, nbins = c->nbins;
+    const double *offs = c->offsets.as<double>();
+    const double g0 = c->p.gate_start, g1 = c->p.gate_stop;
+    int16_t *bins = c->bins.as<int16_t>();
+    cudaStream_t st3 = c->st3;
+    q.wait(st3, sl.deps[0]);
+    q.kernel([=] {
+      launch_pulsar_bins(nrows, K, psr_start_phase, psr_rate, fft_duration, offs, g0, g1, nbins, bins, st3);
+    });
+    c->bins_rows = nrows;
+    launches += 1;
+    if (tc_x) {
+      const int list_len = max_rows + 16 * nbins;
+      int *rowlist = c->rowlist.as<int>();
+      int2 *segs = c->segs.as<int2>();
+      q.kernel([=] { launch_pulsar_sort(bins, nrows, K, nbins, list_len, rowlist, segs, st3); });
+      launches += 1;
+    }
+  }
   size_t ev = 0;
   // Chunk ch's X-step runs on the third stream beside chunk ch + 1's F-step
   // (an X-step CTA and an F-step CTA fit an SM together); chunk ch + 1's
@@ -1178,25 +1201,17 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
       if (c->phased) {
         q.kernel([=] { launch_phased(static_cast<float2 *>(specp), max_rows, kpad, N, r0c, nrows, K, nsub, acc, xs); });
       } else if (pulsar) {
-        // the bin of every (row, channel), then the binned X-step: tensor cores
-        // over each channel's rows sorted by bin, or CUDA cores in row order
-        const double *offs = c->offsets.as<double>();
-        const double g0 = c->p.gate_start, g1 = c->p.gate_stop;
-        int16_t *bins = c->bins.as<int16_t>();
-        q.kernel([=] {
-          launch_pulsar_bins(nrows, K, psr_start_phase, psr_rate, fft_duration, offs, g0, g1, nbins, bins, xs);
-        });
-        c->bins_rows = nrows;  // one chunk: the whole integration
+        // the binned X-step: tensor cores over each channel's rows sorted by
+        // bin, or CUDA cores in row order
+        const int16_t *bins = c->bins.as<int16_t>();
         if (tc_x) {
           const int list_len = max_rows + 16 * nbins;
-          int *rowlist = c->rowlist.as<int>();
-          int2 *segs = c->segs.as<int2>();
-          q.kernel([=] { launch_pulsar_sort(bins, nrows, K, nbins, list_len, rowlist, segs, xs); });
+          const int *rowlist = c->rowlist.as<int>();
+          const int2 *segs = c->segs.as<int2>();
           q.op([=] {
             return launch_xcorr_tc_gather(specp, tc_slots, nrows, kpad, K, N, blmap, npad, nbl, nbins, rowlist,
                                           list_len, segs, inv_s2, acc, derr, xs);
           });
-          launches += 1;
         } else {
           q.kernel([=] {
             launch_xcorr_f32_binned(static_cast<float2 *>(specp), max_rows, kpad, N, npad, nrows, K, tiles, ntiles, blmap,
@@ -1243,7 +1258,7 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
       q.record(sl.deps[1 + ch + 1], c->st2);
     }
     ev += 5;
-    launches += pulsar ? 5 : 4;  // parameters, blocks, window FFT, (pulsar bins,) X-step
+    launches += 4;  // parameters, blocks, window FFT, X-step
   }
   {  // the last chunk, for the autotuner
     sfxc_gpu_ctx::TuneSpec &ts = c->tune;

@@ -772,12 +772,17 @@ __global__ void __launch_bounds__(384, 1) xcorr_f32_kernel(const __grid_constant
 // Pulsar bins (Correlation_core_pulsar::dedisperse_buffer) in FP64, evaluated
 // with the reference's operation order so that every bin matches; written
 // [channel][row] (row fastest) for the per-channel sort and the binned X-steps.
-__global__ void pulsar_bins_kernel(int nrows, int K, double start_phase, double rate_term, double fft_duration,
-                                   const double *__restrict__ offsets, double g0, double g1, int nbins,
-                                   int16_t *__restrict__ bins) {
+// A thread per row takes kBinChans channels: the row's own phase (a division)
+// is computed once for all of them, and the division by the gate's length is
+// left out when that is 1, where it changes nothing.  Bound by the FP64 pipe:
+// 16 M bins 1.83 -> 1.19 ms, and it runs
+// beside the F-step.
+constexpr int kBinChans = 16;
+__global__ void __launch_bounds__(128) pulsar_bins_kernel(int nrows, int K, double start_phase, double rate_term,
+                                                          double fft_duration, const double *__restrict__ offsets,
+                                                          double g0, double g1, int nbins, int16_t *__restrict__ bins) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  const int k = blockIdx.y;
-  if (k >= K || r >= nrows) return;
+  if (r >= nrows) return;
   const double us_per_day = 86400000000.0;
   // start_phase + (coef[1] + 60 F0) * fft_duration * current_fft * 1440 / us_per_day
   double ph = __dmul_rn(rate_term, fft_duration);
@@ -785,18 +790,21 @@ __global__ void pulsar_bins_kernel(int nrows, int K, double start_phase, double 
   ph = __dmul_rn(ph, 1440.0);
   ph = __ddiv_rn(ph, us_per_day);
   ph = __dadd_rn(start_phase, ph);
-  double p = __dsub_rn(ph, offsets[k]);
-  p = __dsub_rn(p, floor(p));
-  const double len = __dsub_rn(g1, g0);
-  int bin;
-  if (p >= g0) {
-    bin = p < g1 ? (int)__ddiv_rn(__dmul_rn(__dsub_rn(p, g0), (double)(nbins - 1)), len) + 1 : 0;
-  } else if (__dadd_rn(p, 1.0) < g1) {
-    bin = (int)__ddiv_rn(__dmul_rn(__dsub_rn(__dadd_rn(p, 1.0), g0), (double)(nbins - 1)), len) + 1;
-  } else {
-    bin = 0;
+  const double len = __dsub_rn(g1, g0), scale = (double)(nbins - 1);
+  const bool whole = len == 1.0;
+  const int k1 = min(K, (int)(blockIdx.y + 1) * kBinChans);
+  for (int k = blockIdx.y * kBinChans; k < k1; k++) {
+    double p = __dsub_rn(ph, __ldg(offsets + k));
+    p = __dsub_rn(p, floor(p));
+    const double p1 = __dadd_rn(p, 1.0);
+    int bin = 0;
+    if (p >= g0 ? p < g1 : p1 < g1) {
+      double x = __dmul_rn(__dsub_rn(p >= g0 ? p : p1, g0), scale);
+      if (!whole) x = __ddiv_rn(x, len);
+      bin = (int)x + 1;
+    }
+    bins[(int64_t)k * nrows + r] = (int16_t)bin;
   }
-  bins[(int64_t)k * nrows + r] = (int16_t)bin;
 }
 
 // ------------------------------------------------------------------------
@@ -1216,8 +1224,8 @@ void launch_xcorr_f32_binned(const float2 *spec, int nrows_total, int kpad, int 
 
 void launch_pulsar_bins(int nrows, int K, double start_phase, double rate_term, double fft_duration,
                         const double *offsets, double g0, double g1, int nbins, int16_t *bins, cudaStream_t st) {
-  pulsar_bins_kernel<<<dim3((nrows + 127) / 128, K), 128, 0, st>>>(nrows, K, start_phase, rate_term, fft_duration,
-                                                                  offsets, g0, g1, nbins, bins);
+  pulsar_bins_kernel<<<dim3((nrows + 127) / 128, (K + kBinChans - 1) / kBinChans), 128, 0, st>>>(
+      nrows, K, start_phase, rate_term, fft_duration, offsets, g0, g1, nbins, bins);
 }
 
 void launch_normalize(const float2 *acc, int kpad, int M, int nstreams, int nbl, int nout, const int *bl, double *norms,

@@ -20,25 +20,31 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
 
 // SM100 shared-memory matrix descriptor: start >> 4 (bits 0-13), leading
 // byte offset >> 4 (16-29), stride byte offset >> 4 (32-45), version 1
-// (bit 46), base offset 0, layout type SWIZZLE_32B = 6 (bits 61-63).  For an
-// MN-major operand the leading offset steps between MN atoms (16 FP16
-// components x 8 K rows = 256 B), the stride offset between 8-row K groups.
+// (bit 46), base offset 0, layout type SWIZZLE_128B = 2 (bits 61-63).  For an
+// MN-major operand the leading offset steps between MN atoms (64 FP16
+// components x 8 K rows = 1 KB, on a 1 KB boundary), the stride offset between
+// 8-row K groups.
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
   uint64_t d = 0;
   d |= (uint64_t)((addr >> 4) & 0x3FFF);
   d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
   d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
   d |= (uint64_t)1 << 46;
-  d |= (uint64_t)6 << 61;
+  d |= (uint64_t)2 << 61;
   return d;
 }
 
-// Byte offset of 16-byte chunk `chunk` (0 or 1) of K row `r` (0..7) inside a
-// 32-byte-swizzled atom of 8 rows x 32 bytes that starts on a 256-byte
-// boundary: the swizzle exchanges the two halves of rows 4..7 (address bit 4
-// XOR address bit 7).
-__host__ __device__ __forceinline__ uint32_t sw32_offset(int r, int chunk) {
-  return (uint32_t)(r * 32 + ((chunk ^ (r >> 2)) & 1) * 16);
+// The same for layout type SWIZZLE_32B = 6: MN atoms of 16 FP16 components x 8
+// K rows = 256 B, what TMA boxes with 32-byte rows produce.
+__device__ __forceinline__ uint64_t smem_desc32(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+  return (smem_desc(addr, lbo, sbo) & ~((uint64_t)7 << 61)) | (uint64_t)6 << 61;
+}
+
+// Byte offset of 16-byte chunk `chunk` (0..7) of K row `r` in a run of 128-byte
+// swizzled rows that starts on a 1 KB boundary: the chunk's number XOR the
+// row's low three bits.
+__host__ __device__ __forceinline__ uint32_t sw128_offset(int r, int chunk) {
+  return (uint32_t)(r * 128 + ((chunk ^ r) & 7) * 16);
 }
 
 // Instruction descriptor, kind::f16: D FP32 (bits 4-5 = 1), A and B FP16
@@ -62,7 +68,7 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 // wall time (and after kSpinLimit polls), returning false.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
   const uint32_t a = smem_u32(bar);
-  const uint64_t t0 = globaltimer_ns();
+  uint64_t t0 = 0;  // first read after 256 polls: a read takes longer than most waits
   for (unsigned long long i = 0; i < kSpinLimit; i++) {
     uint32_t done;
     asm volatile(
@@ -71,7 +77,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
         : "r"(a), "r"(parity)
         : "memory");
     if (done) return true;
-    if ((i & 255) == 255 && globaltimer_ns() - t0 > kWaitNs) return false;
+    if ((i & 255) == 255) {
+      const uint64_t t = globaltimer_ns();
+      if (t0 == 0) t0 = t;
+      if (t - t0 > kWaitNs) return false;
+    }
   }
   return false;
 }

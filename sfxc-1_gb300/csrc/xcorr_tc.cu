@@ -10,9 +10,10 @@
 // 128-byte line per (group of four channels, slot quad), so a channel's
 // slots are eight 32-byte pieces 128 B apart.  One TMA box per channel and
 // K-tile gathers them, with the 32-byte swizzle, into the canonical MN-major
-// layout: atoms of 8 rows x 32 B (16 components), the eight M atoms 256 B
-// apart, 8-row groups 2 KB apart.  The M index of a component is
-// 4 * stream + {hi.re, hi.im, lo.re, lo.im}.  The MMA computes
+// layout: atoms of 8 rows x 32 B (16 components), the nq M atoms 256 B
+// apart, 8-row groups 256 nq bytes apart.  The M index of a component is
+// 4 * stream + {hi.re, hi.im, lo.re, lo.im}.  Only the slot quads that hold
+// streams are loaded (24 streams, 16384 channels, 0.5 s: 1.74 -> 1.45 ms).  The MMA computes
 // D = A A^T (128 x 128, FP32 accumulation in TMEM); summing the four hi/lo
 // combinations of a stream pair gives the compensated product, and the
 // epilogue forms
@@ -20,8 +21,8 @@
 // with lane shuffles over the 4 TMEM lanes (D rows) of one stream.
 //
 // Persistent CTA per SM, 10 warps, warp-specialised, over groups of 2
-// channels: warp 0 streams K-tiles with TMA (cp.async.bulk.tensor, 128-byte
-// swizzle, 2 boxes of 16 KB per 32 KB stage, 4 stages) without stopping at
+// channels: warp 0 streams K-tiles with TMA (cp.async.bulk.tensor, 32-byte
+// swizzle, 2 boxes of 2 KB x nq per stage, 4 to 8 stages) without stopping at
 // group boundaries; warp 1 issues 2 channels x 4 MMAs (K = 16) per stage into
 // one of two TMEM buffers (2 x 256 columns) and commits each stage to its
 // "empty" barrier and each finished group to the buffer's "full" barrier;
@@ -46,13 +47,12 @@ using namespace tc;
 
 constexpr int kChan = 2;        // channels per group (one TMEM buffer)
 constexpr int kRowsK = 64;      // FFT rows per K-tile
-constexpr int kStages = 4;   // 129 KB of shared memory; 3 stages measured 17 % slower, 6 stages 3 %
+constexpr int kMaxStages = 8;
+constexpr int kStagesBytes = 131072;  // the stage ring (4 stages of 32 streams; 3 measured 17 % slower, 6 stages 3 %)
 constexpr int kThreads = 320;   // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
-constexpr int kChanTile = kRowsK * 256;       // one channel's K-tile: 64 rows x 128 components x 2 B
-constexpr int kStageBytes = kChan * kChanTile;  // 32 KB per stage
 constexpr uint32_t kBufCols = kChan * 128;      // TMEM columns per buffer
-// One channel's K-tile: TMA box {16 components, 8 rows, 8 slot quads, 8 row
-// groups, 1 channel group} = 16 KB at row group rg and channel group cg.
+// One channel's K-tile: TMA box {16 components, 8 rows, nq slot quads, 8 row
+// groups, 1 channel group} = 2 KB x nq at row group rg and channel group cg.
 __device__ __forceinline__ void tma_load_tile(void *dst, const CUtensorMap *map, int rg, int cg, uint64_t *bar) {
   tma_load_5d(dst, map, 0, 0, 0, rg, cg, bar);
 }
@@ -63,16 +63,18 @@ struct TcMaps {
 };
 
 __global__ void __launch_bounds__(kThreads, 1)
-    xcorr_tc_kernel(const __grid_constant__ TcMaps tmaps, int nrows, int K, int kpad, const int *__restrict__ blmap,
-                    int npad, float inv_scale2, float2 *__restrict__ acc, int *__restrict__ err) {
+    xcorr_tc_kernel(const __grid_constant__ TcMaps tmaps, int nrows, int K, int kpad, int nq, int nst,
+                    const int *__restrict__ blmap, int npad, float inv_scale2, float2 *__restrict__ acc, int *__restrict__ err) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *base = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);  // stages 1 KB aligned
-  __shared__ uint64_t full[kStages], empty[kStages], tfull[2], tempty[2], done;
+  __shared__ uint64_t full[kMaxStages], empty[kMaxStages], tfull[2], tempty[2], done;
   __shared__ uint32_t tmem_base;
   __shared__ int failed;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ngroups = (K + kChan - 1) / kChan;
   const int nkt = (nrows + kRowsK - 1) / kRowsK;
+  // one channel's K-tile (64 rows x 16 nq components x 2 B) and a stage of two
+  const int ctile = kRowsK * 32 * nq, sbytes = kChan * ctile;
   // this CTA's groups: blockIdx.x, blockIdx.x + gridDim.x, ...
   const int my_groups = blockIdx.x < ngroups ? (ngroups - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
 
@@ -80,7 +82,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     tmem_alloc(&tmem_base, 512);
   }
   if (tid == 0) {
-    for (int s = 0; s < kStages; s++) {
+    for (int s = 0; s < kMaxStages; s++) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
@@ -100,33 +102,30 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   if (tid == 0) {
     // ---- TMA producer: every K-tile of every group, one stage ring
-    int last[kStages];
-    for (int s = 0; s < kStages; s++) last[s] = -1;
     int it = 0;
     for (int i = 0; i < my_groups && !*vfailed; i++) {
       const int g = blockIdx.x + i * gridDim.x;
       for (int kt = 0; kt < nkt; kt++, it++) {
-        const int s = it % kStages, n = it / kStages;
+        const int s = it % nst, n = it / nst;
         if ((n > 0 && !mbar_wait(&empty[s], (n - 1) & 1)) || *vfailed) {
           *vfailed = 1;
           break;
         }
-        mbar_expect_tx(&full[s], kStageBytes);
-        uint8_t *st = base + s * kStageBytes;
+        mbar_expect_tx(&full[s], sbytes);
+        uint8_t *st = base + s * sbytes;
 #pragma unroll
         for (int c = 0; c < kChan; c++) {
           const int ch = g * kChan + c;
-          tma_load_tile(st + c * kChanTile, &tmaps.m[ch & 3], kt * (kRowsK / 8), ch >> 2, &full[s]);
+          tma_load_tile(st + c * ctile, &tmaps.m[ch & 3], kt * (kRowsK / 8), ch >> 2, &full[s]);
         }
-        last[s] = it;
       }
     }
-    // loads still in flight land before the CTA may exit
-    for (int s = 0; s < kStages; s++)
-      if (last[s] >= 0 && !mbar_wait(&full[s], (last[s] / kStages) & 1)) *vfailed = 1;
+    // loads still in flight (the last nst tiles) land before the CTA may exit
+    for (int i = it > nst ? it - nst : 0; i < it; i++)
+      if (!mbar_wait(&full[i % nst], (i / nst) & 1)) *vfailed = 1;
   } else if (tid == 32) {
     // ---- MMA issuer
-    const uint32_t idesc = idesc_f16(128, 128);
+    const uint32_t idesc = idesc_f16(128, 16 * nq);
     int it = 0;
     for (int i = 0; i < my_groups && !*vfailed; i++) {
       const int b = i & 1, u = i >> 1;
@@ -137,19 +136,19 @@ __global__ void __launch_bounds__(kThreads, 1)
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       bool ok = true;
       for (int kt = 0; kt < nkt; kt++, it++) {
-        const int s = it % kStages, n = it / kStages;
+        const int s = it % nst, n = it / nst;
         if (!mbar_wait(&full[s], n & 1)) {
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t st = smem_u32(base + s * kStageBytes);
+        const uint32_t st = smem_u32(base) + s * sbytes;
 #pragma unroll
         for (int c = 0; c < kChan; c++) {
 #pragma unroll
           for (int ks = 0; ks < kRowsK / 16; ks++) {
-            // 16 K-rows = two 8-row groups of 2 KB; M atoms 256 B apart
-            const uint64_t d = smem_desc(st + c * kChanTile + ks * 4096, 256, 2048);
+            // 16 K-rows = two 8-row groups of nq atoms; M atoms 256 B apart
+            const uint64_t d = smem_desc32(st + c * ctile + ks * 512 * nq, 256, 256 * nq);
             mma_f16(tmem + b * kBufCols + c * 128, d, d, idesc, (kt > 0 || ks > 0) ? 1u : 0u);
           }
         }
@@ -176,7 +175,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int k = (blockIdx.x + i * gridDim.x) * kChan + c;
 #pragma unroll 1
-      for (int j = 0; j < 4; j++) {
+      for (int j = 0; 2 * j < nq && 8 * q < npad; j++) {
         float v[32];
         tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + b * kBufCols + c * 128 + j * 32, v);
         float re8[8], im8[8];
@@ -235,28 +234,50 @@ __global__ void __launch_bounds__(kThreads, 1)
 //   * pulsar binning (Correlation_core_pulsar::integration_step,
 //     sfxc/src/correlation_core_pulsar.cc:101-146 with the bins of 210-238):
 //     each channel's rows sorted by bin (pulsar_sort_kernel), one segment per
-//     bin, the segment's Gram added to acc[bin];
+//     bin, the segment's Gram stored as acc[bin];
 //   * jobs of 33 to 64 streams (S = 64 slots): rows in order, one segment.
-// Warps 0-3 gather K-tiles of up to 64 listed rows with 16-byte cp.async
-// straight into the 32-byte-swizzled MN-major layout that the TMA kernel's
-// boxes produce (list entries of -1 read as zero rows) and publish each tile
-// after a proxy fence; warp 4 issues the MMAs -- per 16 rows, block I = 0
+// A tile is up to kRows listed rows of one segment.  Warps 0-3 take the tiles
+// in turn: each copies its tile's rows with 16-byte cp.async, only the slot
+// quads that hold streams, straight into 128-byte-swizzled MN-major atoms of
+// 64 components (list entries of -1 read as zero rows),
+// and publishes it after a proxy fence when its next tile is on the way, so
+// eight tiles are in flight.  Warp 4 issues the MMAs -- per 16 rows, block I = 0
 // (and 1 for S = 64): M = 128 rows of components from 128 I, N = the
 // components from 128 I to the last stream (FP32 accumulation in the
-// segment's TMEM buffer); warps 5-12 add each finished buffer to its
-// accumulator while the next segments accumulate in the other buffers.
+// segment's TMEM buffer; the rows of M past the last stream are whatever lies
+// behind the tile and are not read back).  The remaining warps bring each
+// finished buffer to its accumulator while the next segments accumulate in
+// the other buffers: for S = 32 four warps per TMEM lane quarter, each taking
+// every fourth segment; for S = 64 two, each taking every other 16 columns.
+// Only the producers follow the row list: the tile's place goes through
+// shared memory to the MMA warp and the segment's from there to the epilogue.
 // Every wait is bounded: on timeout the CTA records an error and stops,
 // waits (bounded) for its copies and MMAs in flight, frees its TMEM and
 // returns.
+//
+// Bound: with binning, the chains of small steps a segment of few rows takes
+// in each role (copies about 700 cycles a segment and warp, MMA issue and its
+// commits 700, epilogue 1300 over four sets): 526,000 (channel, bin) segments
+// of 30 rows of 20 streams 6.36 -> 2.87 ms.  Copying chunk by chunk instead of
+// four at a time, to overlap their shuffles and addresses, takes 3.8 ms, eight
+// at a time 3.1; 32-byte-swizzled atoms 3.85 against 3.79 then.  For 33 to 64
+// streams, L2 and DRAM reads of 32-byte pieces: 40 streams, 4096 channels,
+// 1953 rows 2.57 -> 0.82 ms (3.1 TB/s of spectra) -- slot quads without streams
+// were read too, and a CTA took the four channels of a group one after the
+// other, by when their common 128-byte lines had left L2 (6.4 TB/s from DRAM
+// for 1.6 of spectra); now four CTAs take them at the same time.
 template <int S>
 struct GatherShape {
-  static constexpr int kRows = 64;                       // rows per K-tile
-  static constexpr int kGroupBytes = (S / 4) * 256;      // one 8-row K group: S/4 atoms of 8 rows x 32 B
-  static constexpr int kStageBytes = 8 * kGroupBytes;    // 16 KB (S = 32) or 32 KB (S = 64)
-  static constexpr int kStages = 131072 / kStageBytes;   // 128 KB of stages: one CTA per SM
-  static constexpr int kProducers = 128;                 // warps 0-3
-  static constexpr int kThreads = 416;                   // + warp 4 (MMA) + warps 5-12 (epilogue)
-  static constexpr size_t kSmem = (size_t)kStages * kStageBytes + 1024;
+  static constexpr int kRows = S == kTcSlots ? 64 : 32;  // rows per tile (at most 16 KB)
+  static constexpr int kStagesBytes = 131072;            // the stage ring: one CTA per SM
+  static constexpr int kMaxStages = 16;
+  static constexpr int kProducers = 4;                   // warps 0-3
+  static constexpr int kSets = S == kTcSlots ? 4 : 2;    // epilogue warps per TMEM lane quarter
+  static constexpr bool kBySegment = S == kTcSlots;      // the sets take whole segments in turn
+  static constexpr int kSlots = S == kTcSlots ? 8 : 12;  // 16-column chunks per epilogue warp and segment
+  static constexpr int kThreads = 32 * (kProducers + 1 + 4 * kSets);
+  // + alignment + what M = 128 reads behind the last stage (one atom column)
+  static constexpr size_t kSmem = kStagesBytes + 1024 + kRows * 128;
 };
 
 struct GatherArgs {
@@ -270,6 +291,8 @@ struct GatherArgs {
   float inv_scale2;
   float2 *acc;          // [bin][baseline][kpad]
   int *err;
+  int nq, nst;          // slot quads with streams; stages of the ring
+  int parts, part_bins; // units of work: channel groups of four x parts of the bins (a multiple of 8 bins each)
   int n0, n1, col1;     // MMA N of blocks 0 and 1 (n1 = 0: one block), TMEM column of block 1
   int buf_stride, nbuf; // TMEM columns per buffer, number of buffers
   int accumulate;       // 0: every (bin, channel) segment is the only one of its launch and is stored as it is
@@ -277,61 +300,79 @@ struct GatherArgs {
 
 constexpr int kMaxBufs = 8;
 
-__device__ __forceinline__ int2 gather_seg(const GatherArgs &g, int ch, int bin) {
-  if (!g.segs) return make_int2(0, (g.nrows + 15) & ~15);
-  return g.segs[(size_t)ch * g.nbins + bin];
-}
-
-// One K-tile of a segment.
-struct GTile {
-  int ch, bin, e0, rows;  // channel, bin, first list entry, rows (a multiple of 16)
-  bool first, last;       // first / last tile of its segment
-};
-
-// The K-tiles of this CTA in processing order: channel groups of four
-// (group blockIdx.x, then + gridDim.x); within a group bin by bin; within a
-// bin the group's four channels; within a segment 64 rows at a time.  The
-// four channels of a group read the four 32-byte pieces of the same 128-byte
-// spectra lines and write the same 32-byte accumulator sectors close together
-// in time.  Every role of the kernel walks the same sequence.
+// The tiles of this CTA in processing order: its units (unit blockIdx.x, then
+// + gridDim.x) of a group of four channels and a part of the bins; within a
+// unit bin by bin; within a bin the group's four channels; within a segment R
+// rows at a time.  The four channels of a group read the four 32-byte pieces
+// of the same 128-byte spectra lines and write the same 32-byte accumulator
+// sectors close together in time.  Warp-wide: lane l holds the segment of
+// (bin, channel) number kb + l of the unit, and that of kb + 32 + l is on its way.
 struct GWalk {
-  int grp, bin, c, t0;
-  int2 sg;
-  __device__ void init() {
-    grp = blockIdx.x;
-    bin = 0;
-    c = -1;
-    t0 = 0;
-    sg = make_int2(0, 0);
+  int u, nunits, grp, kb, kend, cur, e0, len, t0, lane;
+  int2 seg, next_seg;
+  unsigned mask;
+  __device__ int2 load(const GatherArgs &g, int k) const {
+    const int ch = 4 * grp + (k & 3);
+    if (k >= kend || ch >= g.K) return make_int2(0, 0);
+    return g.segs ? __ldg(g.segs + (size_t)ch * g.nbins + (k >> 2)) : make_int2(0, (g.nrows + 15) & ~15);
   }
-  __device__ bool next(const GatherArgs &g, int ngroups, GTile &t) {
-    if (t0 + 64 < sg.y) {  // more rows in the current segment
-      t0 += 64;
-    } else {
-      for (;;) {  // the next non-empty segment
-        if (++c == 4) {
-          c = 0;
-          if (++bin == g.nbins) {
-            bin = 0;
-            grp += gridDim.x;
-          }
-        }
-        if (grp >= ngroups) return false;
-        const int ch = 4 * grp + c;
-        if (ch >= g.K) continue;
-        sg = gather_seg(g, ch, bin);
-        if (sg.y > 0) break;
-      }
-      t0 = 0;
+  __device__ void unit(const GatherArgs &g) {
+    grp = u / g.parts;
+    const int part = u - grp * g.parts;
+    kb = g.segs ? 4 * part * g.part_bins : part;
+    kend = g.segs ? min(4 * g.nbins, kb + 4 * g.part_bins) : part + 1;
+    next_seg = load(g, kb + lane);
+  }
+  __device__ void batch(const GatherArgs &g) {
+    seg = next_seg;
+    next_seg = load(g, kb + 32 + lane);
+    mask = __ballot_sync(0xffffffffu, seg.y > 0);
+    cur = -1;
+  }
+  __device__ void init(const GatherArgs &g) {
+    lane = threadIdx.x & 31;
+    nunits = (g.K + 3) / 4 * g.parts;
+    u = blockIdx.x;
+    cur = -1;
+    len = t0 = 0;
+    mask = 0;
+    kb = kend = 0;
+    if (u < nunits) {
+      unit(g);
+      batch(g);
     }
-    t.ch = 4 * grp + c;
-    t.bin = bin;
-    t.e0 = sg.x + t0;
-    t.rows = min(64, sg.y - t0);
-    t.first = t0 == 0;
-    t.last = t0 + 64 >= sg.y;
+  }
+  // the next tile: e0 + t0 its first list entry
+  __device__ bool next(const GatherArgs &g, int R) {
+    t0 += R;
+    if (t0 < len) return true;
+    for (;;) {
+      const unsigned rest = mask & (cur < 0 ? ~0u : ~1u << cur);
+      if (rest) {
+        cur = __ffs(rest) - 1;
+        break;
+      }
+      if (u >= nunits) return false;
+      kb += 32;
+      if (kb >= kend) {
+        u += gridDim.x;
+        mask = 0;
+        if (u >= nunits) return false;
+        unit(g);
+      }
+      batch(g);
+    }
+    e0 = __shfl_sync(0xffffffffu, seg.x, cur);
+    len = __shfl_sync(0xffffffffu, seg.y, cur);
+    t0 = 0;
     return true;
   }
+};
+
+// A tile in the ring: rows (a multiple of 16; -1: no more tiles), channel,
+// bin, bit 0 / 1: first / last of its segment.
+struct GTile {
+  int rows, ch, bin, flags;
 };
 
 template <int S>
@@ -339,19 +380,21 @@ __global__ void __launch_bounds__(GatherShape<S>::kThreads, 1) xcorr_tc_gather_k
   using G = GatherShape<S>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *base = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);  // stages 1 KB aligned
-  __shared__ uint64_t full[G::kStages], empty[G::kStages], tfull[kMaxBufs], tempty[kMaxBufs], done;
+  __shared__ uint64_t full[G::kMaxStages], empty[G::kMaxStages], tfull[kMaxBufs], tempty[kMaxBufs], done;
+  __shared__ GTile tiles[G::kMaxStages];
+  __shared__ int2 segs[kMaxBufs];  // channel (-1: no more segments) and bin of each TMEM buffer
   __shared__ uint32_t tmem_base;
   __shared__ int failed;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (warp == 4) tmem_alloc(&tmem_base, 512);
   if (tid == 0) {
-    for (int s = 0; s < G::kStages; s++) {
-      mbar_init(&full[s], G::kProducers);
+    for (int s = 0; s < G::kMaxStages; s++) {
+      mbar_init(&full[s], 32);
       mbar_init(&empty[s], 1);
     }
     for (int b = 0; b < kMaxBufs; b++) {
-      mbar_init(&tfull[b], 1);
-      mbar_init(&tempty[b], 8);  // one arrival per epilogue warp
+      mbar_init(&tfull[b], 2);  // the MMAs' commit and the issuer
+      mbar_init(&tempty[b], G::kBySegment ? 4 : 4 * G::kSets);  // one arrival per epilogue warp of the segment
     }
     mbar_init(&done, 1);
     failed = 0;
@@ -362,175 +405,244 @@ __global__ void __launch_bounds__(GatherShape<S>::kThreads, 1) xcorr_tc_gather_k
   fence_after_sync();
   const uint32_t tmem = tmem_base;
   volatile int *vfailed = &failed;
-  const int ngroups = (g.K + 3) / 4;
-  GWalk walk;
-  walk.init();
-  GTile t;
+  constexpr int kAtoms = G::kRows * 128;         // a column of atoms: kRows rows x 64 components
+  const int sbytes = (g.nq + 3) / 4 * kAtoms;    // one stage
 
-  if (tid < G::kProducers) {
-    // ---- producers: thread tid copies, for every row j = j0 + RP i of a
-    // tile, the 16-byte half h of slot quad q (quads one 128-byte line
-    // apart); the row-list entries of the next tile load while the current
-    // tile is issued
-    constexpr int CPR = S / 2;               // 16-byte chunks per row
-    constexpr int RP = G::kProducers / CPR;  // rows per pass
-    constexpr int E = G::kRows / RP;         // rows per thread and tile
-    const int j0 = tid / CPR, q = (tid % CPR) >> 1, h = tid & 1;
-    const uint32_t soff = q * 256;
+  if (warp < G::kProducers) {
+    // ---- producers: tile it is warp it % 4's; its rows' 16-byte chunks (2 nq
+    // a row) lane by lane; the list entries of the warp's next tile load while
+    // the current one is issued
+    constexpr int E = G::kRows / 32, U = 4;
+    const int cpr = 2 * g.nq, dj = 32 / cpr, dc = 32 % cpr, j0 = lane / cpr, c0 = lane % cpr;
     const int64_t rstride = (int64_t)g.kpad * S * 8;  // bytes per row
-    int rcur[E], rnxt[E];
-    auto load_rows = [&](const GTile &x, int(&r)[E]) {
-      const int *list = g.rowlist ? g.rowlist + (size_t)x.ch * g.list_len : nullptr;
-#pragma unroll
-      for (int i = 0; i < E; i++) {
-        const int j = j0 + RP * i;
-        r[i] = j < x.rows ? (list ? __ldg(list + x.e0 + j) : x.e0 + j) : -2;
+    GWalk walk;
+    walk.init(g);
+    int it = -1;  // the tile the walk stands at
+    struct Mine {
+      GTile t;
+      int row[E];
+    } cur, nxt;
+    auto advance = [&](int steps, Mine &m) -> bool {  // to the warp's next tile; false: `it` is the number of tiles
+      for (int i = 0; i < steps; i++) {
+        it++;
+        if (!walk.next(g, G::kRows)) return false;
       }
+      m.t.rows = min(G::kRows, walk.len - walk.t0);
+      m.t.ch = 4 * walk.grp + ((walk.kb + walk.cur) & 3);
+      m.t.bin = (walk.kb + walk.cur) >> 2;
+      m.t.flags = (walk.t0 == 0 ? 1 : 0) | (walk.t0 + G::kRows >= walk.len ? 2 : 0);
+      const int e = walk.e0 + walk.t0 + lane;
+#pragma unroll
+      for (int i = 0; i < E; i++)
+        m.row[i] = !g.rowlist ? e + 32 * i
+                   : lane + 32 * i < m.t.rows ? __ldg(g.rowlist + (size_t)m.t.ch * g.list_len + e + 32 * i) : -1;
+      return true;
     };
-    GTile cur, nxt;
-    bool have = walk.next(g, ngroups, cur);
-    if (have) load_rows(cur, rcur);
-    int it = 0;
+    auto publish = [&](int tile) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      mbar_arrive(&full[tile % g.nst]);
+    };
+    bool have = advance(warp + 1, cur);
+    int mine = it, last = -1;
+    bool ok = true;
     while (have) {
-      const bool have_next = walk.next(g, ngroups, nxt);
-      if (have_next) load_rows(nxt, rnxt);
-      const int s = it % G::kStages, n = it / G::kStages;
-      if ((n > 0 && !mbar_wait(&empty[s], (n - 1) & 1)) || *vfailed) {
-        *vfailed = 1;
-        break;
-      }
-      const uint32_t st = smem_u32(base + s * G::kStageBytes);
-      const uint8_t *chbase = g.spec + (tc_index(0, g.kpad, cur.ch, 4 * q, S) * 8 + 16 * h);
+      const bool have_next = advance(4, nxt);
+      const int s = mine % g.nst, n = mine / g.nst;
+      ok = __all_sync(0xffffffffu, (n == 0 || mbar_wait(&empty[s], (n - 1) & 1)) && !*vfailed);
+      if (!ok) break;
+      if (lane == 0) tiles[s] = cur.t;
+      const uint32_t st = smem_u32(base) + s * sbytes;
+      const uint8_t *chbase = g.spec + tc_index(0, g.kpad, cur.t.ch, 0, S) * 8;
+      const int total = cur.t.rows * cpr;
+      int j = j0, c = c0;
+      for (int x = lane; x < total + lane; x += 32 * U) {  // U chunks a lane at a time, to overlap their latencies
+        int jj[U], cc[U], row[U];
 #pragma unroll
-      for (int i = 0; i < E; i++) {
-        if (rcur[i] == -2) break;  // past the tile's rows (the rows grow with i)
-        const int j = j0 + RP * i, row = rcur[i];
-        const bool ok = row >= 0 && row < g.nrows;
-        cp_async16(st + (j >> 3) * G::kGroupBytes + soff + sw32_offset(j & 7, h), ok ? chbase + row * rstride : g.spec,
-                   ok ? 16u : 0u);
+        for (int i = 0; i < U; i++) {
+          jj[i] = j;
+          cc[i] = c;
+          j += dj;
+          c += dc;
+          if (c >= cpr) {
+            c -= cpr;
+            j++;
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < U; i++) {
+          row[i] = __shfl_sync(0xffffffffu, cur.row[0], jj[i] & 31);
+          if (E > 1) {
+            const int r1 = __shfl_sync(0xffffffffu, cur.row[E - 1], jj[i] & 31);
+            if (jj[i] >= 32) row[i] = r1;
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < U; i++) {
+          const bool in = (unsigned)row[i] < (unsigned)g.nrows;
+          const uint8_t *src = chbase + (in ? row[i] : 0) * rstride + (cc[i] >> 1) * 128 + (cc[i] & 1) * 16;
+          if (x + 32 * i < total) cp_async16(st + (cc[i] >> 3) * kAtoms + sw128_offset(jj[i], cc[i]), src, in ? 16u : 0u);
+        }
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
-      if (it > 0) {  // the previous tile has landed: publish it to the tensor cores
+      if (last >= 0) {  // the warp's previous tile has landed: publish it to the tensor cores
         asm volatile("cp.async.wait_group 1;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_arrive(&full[(it - 1) % G::kStages]);
+        publish(last);
       }
-      it++;
+      last = mine;
+      mine += 4;
       cur = nxt;
-#pragma unroll
-      for (int i = 0; i < E; i++) rcur[i] = rnxt[i];
       have = have_next;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    if (it > 0) mbar_arrive(&full[(it - 1) % G::kStages]);
+    if (last >= 0) publish(last);
+    if (ok && it % 4 == warp) {  // after the last tile, in its warp's turn: the end
+      const int s = it % g.nst, n = it / g.nst;
+      if (n > 0 && !mbar_wait(&empty[s], (n - 1) & 1)) ok = false;
+      if (lane == 0) tiles[s].rows = -1;
+      mbar_arrive(&full[s]);
+    }
+    if (!ok) *vfailed = 1;
   } else if (tid == 4 * 32) {
     // ---- MMA issuer
     const uint32_t id0 = idesc_f16(128, g.n0), id1 = idesc_f16(128, g.n1 > 0 ? g.n1 : 16);
-    int it = 0, sgn = 0;
+    int s = 0, b = 0, sphase = 0, u = 0;  // stage and its parity, TMEM buffer and its uses
     uint32_t d0 = tmem;
-    while (walk.next(g, ngroups, t)) {
-      const int b = sgn % g.nbuf, u = sgn / g.nbuf;
-      if (t.first) {
-        if ((u > 0 && !mbar_wait(&tempty[b], (u - 1) & 1)) || *vfailed) {  // the epilogue has read buffer b
-          *vfailed = 1;
+    const uint64_t ring = smem_desc(smem_u32(base), kAtoms, 1024);
+    bool ok = true;
+    // buffer b is free: the epilogue has read its previous segment
+    auto claim = [&]() { return (u == 0 || mbar_wait(&tempty[b], (u - 1) & 1)) && !*vfailed; };
+    auto advance = [&]() {
+      if (++b == g.nbuf) {
+        b = 0;
+        u++;
+      }
+    };
+    for (;;) {
+      if (!mbar_wait(&full[s], sphase) || *vfailed) {
+        ok = false;
+        break;
+      }
+      const GTile t = tiles[s];
+      if (t.rows < 0) break;
+      if (t.flags & 1) {
+        if (!claim()) {
+          ok = false;
           break;
         }
-        fence_after_sync();
+        segs[b] = make_int2(t.ch, t.bin);
         d0 = tmem + (uint32_t)(b * g.buf_stride);
       }
-      const int s = it % G::kStages, n = it / G::kStages;
-      if (!mbar_wait(&full[s], n & 1)) {
-        *vfailed = 1;
-        break;
-      }
       fence_after_sync();
-      const uint32_t st = smem_u32(base + s * G::kStageBytes);
-      for (int ks = 0; ks < t.rows / 16; ks++) {
-        const uint32_t acc_flag = (!t.first || ks > 0) ? 1u : 0u;
-        // 16 K rows = two 8-row groups; MN atoms 256 B apart; block 1 starts 8 atoms in
-        const uint64_t a0 = smem_desc(st + ks * 2 * G::kGroupBytes, 256, G::kGroupBytes);
+      uint32_t acc_flag = t.flags & 1 ? 0u : 1u;
+      uint64_t a0 = ring + (uint32_t)((s * sbytes) >> 4);
+#pragma unroll
+      for (int ks = 0; ks < G::kRows / 16; ks++, a0 += 2048 >> 4) {
+        if (ks * 16 >= t.rows) break;
+        // 16 K rows = two 8-row groups of 1 KB; block 1 starts two atoms in
         mma_f16(d0, a0, a0, id0, acc_flag);
-        if (g.n1 > 0) {
-          const uint64_t a1 = smem_desc(st + ks * 2 * G::kGroupBytes + 2048, 256, G::kGroupBytes);
+        if (S > kTcSlots) {
+          const uint64_t a1 = a0 + (2 * kAtoms >> 4);
           mma_f16(d0 + (uint32_t)g.col1, a1, a1, id1, acc_flag);
         }
+        acc_flag = 1u;
       }
       mma_commit(&empty[s]);
-      it++;
-      if (t.last) {
+      if (++s == g.nst) {
+        s = 0;
+        sphase ^= 1;
+      }
+      if (t.flags & 2) {
         mma_commit(&tfull[b]);  // the segment's sums are complete when its MMAs are
-        sgn++;
+        mbar_arrive(&tfull[b]);
+        advance();
       }
     }
+    for (int e = 0; ok && e < (G::kBySegment ? G::kSets : 1); e++) {  // the end, to every set
+      if (!claim()) ok = false;
+      segs[b] = make_int2(-1, 0);
+      mbar_arrive(&tfull[b]);
+      mbar_arrive(&tfull[b]);
+      advance();
+    }
+    if (!ok) *vfailed = 1;
     mma_commit(&done);  // arrives once every MMA issued above has completed
-  } else if (warp >= 5) {
-    // ---- epilogue: warp w reads TMEM lane quarter q = w % 4 (D rows 32 q ..
-    // 32 q + 31 of each block) and every other 16-column chunk
-    const int q = warp & 3, half = (warp - 5) >> 2;
-    const int m = q * 32 + lane, p = m & 3;
-    int sgn = 0;
-    while (walk.next(g, ngroups, t)) {
-      if (!t.last) continue;
-      const int b = sgn % g.nbuf, u = sgn / g.nbuf;
-      if (!mbar_wait(&tfull[b], u & 1) || *vfailed) {
+  } else if (warp > G::kProducers) {
+    // ---- epilogue: a warp reads TMEM lane quarter q = warp % 4 (D rows 32 q ..
+    // 32 q + 31 of each block), in chunks of 16 columns (4 streams).  Lane
+    // 4 i + p of a chunk has component p of row stream 8 q + i (0 hi.re, 1
+    // hi.im, 2 lo.re, 3 lo.im; columns likewise) for the 4 column streams;
+    // the exchange that sums the four components leaves column stream p's sum
+    // in lane p, which stores it.
+    const int q = warp & 3, set = (warp - G::kProducers - 1) >> 2;
+    const int p = lane & 3;
+    int off[G::kSlots];   // accumulator index * 2 + conjugate, per chunk; -1: no such baseline
+    unsigned active = 0;  // chunks with a baseline
+#pragma unroll
+    for (int i = 0; i < G::kSlots; i++) {
+      const int I = i >> 3, chunk = G::kBySegment ? i : 2 * (i & 7) + set;
+      const int a = 32 * I + 8 * q + (lane >> 2), bs = 32 * I + 4 * chunk + p;
+      const int v = a < g.nstreams && bs < g.nstreams && chunk < (I ? g.n1 : g.n0) / 16 ? __ldg(g.blmap + a * g.npad + bs) : -1;
+      off[i] = v < 0 ? -1 : (v >> 1) * g.kpad * 2 + (v & 1);
+      if (__any_sync(0xffffffffu, v >= 0)) active |= 1u << i;
+    }
+    int b = 0, u = 0;
+    auto skip = [&](int n) {
+      for (int i = 0; i < n; i++)
+        if (++b == g.nbuf) {
+          b = 0;
+          u ^= 1;
+        }
+    };
+    if (G::kBySegment) skip(set);
+    for (;;) {
+      if (!__all_sync(0xffffffffu, mbar_wait(&tfull[b], u) && !*vfailed)) {
         *vfailed = 1;
         break;
       }
       fence_after_sync();
-      float2 *accb = g.acc + (size_t)t.bin * g.nbl * g.kpad + t.ch;
-      for (int I = 0; I < (g.n1 > 0 ? 2 : 1); I++) {
-        if (32 * I + 8 * q >= g.nstreams) continue;  // no stream in this lane quarter
-        const int a = 32 * I + (m >> 2);
-        const int nI = I ? g.n1 : g.n0;
-        const uint32_t col = (uint32_t)(b * g.buf_stride + (I ? g.col1 : 0));
-#pragma unroll 1
-        for (int chunk = half; chunk < nI / 16; chunk += 2) {
-          float v[16];
-          tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + col + 16 * chunk, v);
-          float re4[4], im4[4];
+      const int2 sg = segs[b];
+      if (sg.x < 0) break;
+      float2 *accb = g.acc + (size_t)sg.y * g.nbl * g.kpad + sg.x;
 #pragma unroll
-          for (int bb = 0; bb < 4; bb++) {
-            const float A = v[4 * bb] + v[4 * bb + 2], B = v[4 * bb + 1] + v[4 * bb + 3];
-            // row component p: 0 hi.re, 1 hi.im, 2 lo.re, 3 lo.im; columns likewise
-            float re = (p & 1) ? B : A, im = (p & 1) ? A : -B;
-            re += __shfl_xor_sync(0xffffffffu, re, 1);
-            im += __shfl_xor_sync(0xffffffffu, im, 1);
-            re += __shfl_xor_sync(0xffffffffu, re, 2);
-            im += __shfl_xor_sync(0xffffffffu, im, 2);
-            re4[bb] = re;
-            im4[bb] = im;
-          }
-          if (p == 0 && a < g.nstreams) {
-            int mv[4];
+      for (int i = 0; i < G::kSlots; i++) {
+        if (!(active >> i & 1)) continue;
+        const int I = i >> 3, chunk = G::kBySegment ? i : 2 * (i & 7) + set;
+        float2 o = make_float2(0.f, 0.f);
+        float2 *dst = accb + (off[i] >> 1);
+        if (g.accumulate && off[i] >= 0) o = *dst;
+        float v[16];
+        tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * g.buf_stride + (I ? g.col1 : 0) + 16 * chunk), v);
+        float re[4], im[4];
 #pragma unroll
-            for (int bb = 0; bb < 4; bb++) {
-              const int bs = 32 * I + 4 * chunk + bb;
-              mv[bb] = bs < g.nstreams ? __ldg(g.blmap + a * g.npad + bs) : -1;
-            }
-            float2 o[4];
-            if (g.accumulate) {
+        for (int bb = 0; bb < 4; bb++) {
+          const float A = v[4 * bb] + v[4 * bb + 2], B = v[4 * bb + 1] + v[4 * bb + 3];
+          re[bb] = (p & 1) ? B : A;
+          im[bb] = (p & 1) ? A : -B;
+        }
+        // (component p + p ^ 1) + (the other two): lanes keep the column
+        // streams of their own low bit, then of their own high bit
+        float r2[2], i2[2];
 #pragma unroll
-              for (int bb = 0; bb < 4; bb++)
-                if (mv[bb] >= 0) o[bb] = accb[(size_t)(mv[bb] >> 1) * g.kpad];
-            } else {
-#pragma unroll
-              for (int bb = 0; bb < 4; bb++) o[bb] = make_float2(0.f, 0.f);
-            }
-#pragma unroll
-            for (int bb = 0; bb < 4; bb++)
-              if (mv[bb] >= 0) {
-                o[bb].x += re4[bb] * g.inv_scale2;
-                o[bb].y += ((mv[bb] & 1) ? -im4[bb] : im4[bb]) * g.inv_scale2;
-                accb[(size_t)(mv[bb] >> 1) * g.kpad] = o[bb];
-              }
-          }
+        for (int h = 0; h < 2; h++) {
+          const float kr = (p & 1) ? re[2 * h + 1] : re[2 * h], sr = (p & 1) ? re[2 * h] : re[2 * h + 1];
+          const float ki = (p & 1) ? im[2 * h + 1] : im[2 * h], si = (p & 1) ? im[2 * h] : im[2 * h + 1];
+          r2[h] = kr + __shfl_xor_sync(0xffffffffu, sr, 1);
+          i2[h] = ki + __shfl_xor_sync(0xffffffffu, si, 1);
+        }
+        const float kr = (p & 2) ? r2[1] : r2[0], sr = (p & 2) ? r2[0] : r2[1];
+        const float ki = (p & 2) ? i2[1] : i2[0], si = (p & 2) ? i2[0] : i2[1];
+        const float vr = kr + __shfl_xor_sync(0xffffffffu, sr, 2);
+        const float vi = ki + __shfl_xor_sync(0xffffffffu, si, 2);
+        if (off[i] >= 0) {
+          o.x += vr * g.inv_scale2;
+          o.y += ((off[i] & 1) ? -vi : vi) * g.inv_scale2;
+          *dst = o;
         }
       }
       fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[b]);  // buffer b may be overwritten
-      sgn++;
+      skip(G::kBySegment ? G::kSets : 1);
     }
   }
   __syncthreads();
@@ -594,7 +706,8 @@ __global__ void __launch_bounds__(128) pulsar_sort_kernel(const int16_t *__restr
 
 }  // namespace
 
-size_t xcorr_tc_smem_bytes() { return kStages * (size_t)kStageBytes + 1024; }
+// + alignment + what the M = 128 operand reads behind the last stage's last row group
+size_t xcorr_tc_smem_bytes() { return kStagesBytes + 1024 + 2048; }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link
 // against libcuda).
@@ -620,12 +733,13 @@ cudaError_t launch_xcorr_tc(const void *spec, int nrows, int kpad, int K, const 
   // apart), 8-row groups, channel groups (1 KB apart).  Rows from nrows up to
   // the next multiple of 8 must be zero in the buffer (the caller clears
   // them); row groups past the end read as zeros.
-  if (kpad % 4 != 0) return cudaErrorInvalidValue;
+  if (kpad % 4 != 0 || npad % 4 != 0 || npad <= 0 || npad > kTcSlots) return cudaErrorInvalidValue;
   TcMaps maps;
   const cuuint64_t R = (cuuint64_t)kpad * 256;
   const cuuint64_t dims[5] = {16, 8, 8, (cuuint64_t)(nrows + 7) / 8, (cuuint64_t)kpad / 4};
   const cuuint64_t strides[4] = {R, 128, 8 * R, 1024};
-  const cuuint32_t box[5] = {16, 8, 8, (cuuint32_t)kRowsK / 8, 1};
+  const int nq = npad / 4;  // slot quads with streams: only these are read
+  const cuuint32_t box[5] = {16, 8, (cuuint32_t)nq, (cuuint32_t)kRowsK / 8, 1};
   const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
   for (int cc = 0; cc < 4; cc++)
     if (enc(&maps.m[cc], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, static_cast<char *>(const_cast<void *>(spec)) + 32 * cc,
@@ -639,8 +753,9 @@ cudaError_t launch_xcorr_tc(const void *spec, int nrows, int kpad, int K, const 
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm <= 0) nsm = 1;
   const int ngroups = (K + kChan - 1) / kChan;
-  xcorr_tc_kernel<<<std::min(ngroups, nsm), kThreads, smem, st>>>(maps, nrows, K, kpad, blmap, npad, inv_scale2, acc,
-                                                                   err);
+  const int nst = std::min(kMaxStages, kStagesBytes / (kChan * kRowsK * 32 * nq));
+  xcorr_tc_kernel<<<std::min(ngroups, nsm), kThreads, smem, st>>>(maps, nrows, K, kpad, nq, nst, blmap, npad,
+                                                                   inv_scale2, acc, err);
   return cudaGetLastError();
 }
 
@@ -653,7 +768,24 @@ static cudaError_t launch_gather(const GatherArgs &g, cudaStream_t st) {
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm <= 0) nsm = 1;
-  xcorr_tc_gather_kernel<S><<<std::min((g.K + 3) / 4, nsm), G::kThreads, G::kSmem, st>>>(g);
+  const int ngroups = (g.K + 3) / 4;
+  GatherArgs a = g;
+  // a multiple of the producer warps (8 or more), so that a stage is always
+  // the same warp's and that warp sees every phase of its barriers; the same
+  // for the buffers and the epilogue sets that take whole segments (4 or 8)
+  a.nst = std::min(G::kMaxStages, G::kStagesBytes / (G::kRows * 128 * ((a.nq + 3) / 4))) / G::kProducers * G::kProducers;
+  if (G::kBySegment) a.nbuf = a.nbuf / G::kSets * G::kSets;
+  if (a.rowlist) {
+    // parts of the bins (at least 16) so that every CTA has 12 units or more:
+    // the last, partly filled round is then at most a twelfth
+    a.parts = std::max(1, std::min((12 * nsm + ngroups - 1) / ngroups, a.nbins / 16));
+    a.part_bins = a.parts > 1 ? ((a.nbins + a.parts - 1) / a.parts + 7) / 8 * 8 : a.nbins;
+    a.parts = (a.nbins + a.part_bins - 1) / a.part_bins;
+  } else {
+    a.parts = 4;  // one channel a unit
+    a.part_bins = 1;
+  }
+  xcorr_tc_gather_kernel<S><<<std::min(ngroups * a.parts, nsm), G::kThreads, G::kSmem, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -661,7 +793,8 @@ cudaError_t launch_xcorr_tc_gather(const void *spec, int slots, int nrows, int k
                                    const int *blmap, int npad, int nbl, int nbins, const int *rowlist, int list_len,
                                    const int2 *segs, float inv_scale2, float2 *acc, int *err, cudaStream_t st) {
   if (nrows <= 0 || K <= 0) return cudaSuccess;
-  if ((slots != kTcSlots && slots != kTcSlotsWide) || nstreams > slots || nstreams <= 0)
+  // 64 slots only for what 32 do not hold: their second row block is always issued
+  if (nstreams <= 0 || slots != (nstreams <= kTcSlots ? kTcSlots : kTcSlotsWide) || nstreams > kTcSlotsWide)
     return cudaErrorInvalidValue;
   GatherArgs g;
   g.spec = static_cast<const uint8_t *>(spec);
@@ -679,6 +812,7 @@ cudaError_t launch_xcorr_tc_gather(const void *spec, int slots, int nrows, int k
   g.inv_scale2 = inv_scale2;
   g.acc = acc;
   g.err = err;
+  g.nq = (nstreams + 3) / 4;
   auto up16 = [](int x) { return (x + 15) & ~15; };
   auto up32 = [](int x) { return (x + 31) & ~31; };
   const int comps = 4 * nstreams;
