@@ -152,13 +152,6 @@ __device__ __forceinline__ double stream_amplitude(const StreamDev &s, int64_t t
   return spline_eval(s.spline, s.spline_n, 2, time_diff_dev(t, s.scan_begin));
 }
 
-// Barriers for the register FFT (fft_reg.cuh): a warp or the whole CTA.
-struct WarpSync {
-  __device__ void operator()() const { __syncwarp(); }
-};
-struct BlockSync {
-  __device__ void operator()() const { __syncthreads(); }
-};
 // Named barrier `id` (1..15) over `count` threads (a multiple of 32) of the CTA.
 struct GroupSync {
   int id, count;

@@ -174,16 +174,17 @@ struct PackShape {
   }
 };
 
-// The twiddle tables of PackShape<LOGN, NV> from tw[j] = exp(-2 pi i j / N):
+// The twiddle tables of PackShape<LOGN, NV> from tw[j step] = exp(-2 pi i j / N):
 // for each pass, tab[off + (k - 1) (L / NV) + p] = W_L^(p k).
 template <int LOGN, int NV>
-__device__ __forceinline__ void fill_pack_table(float2 *tab, const float2 *__restrict__ tw, int tid, int nthr) {
+__device__ __forceinline__ void fill_pack_table(float2 *tab, const float2 *__restrict__ tw, int tid, int nthr,
+                                                int step = 1) {
   using F = PackShape<LOGN, NV>;
   int off = 0, L = F::N;
 #pragma unroll
   for (int i = 0; i <= F::NMID; i++) {
     const int H = L / NV;
-    for (int e = tid; e < (NV - 1) * H; e += nthr) tab[off + e] = __ldg(tw + (1 + e / H) * (e % H) * (F::N / L));
+    for (int e = tid; e < (NV - 1) * H; e += nthr) tab[off + e] = __ldg(tw + (1 + e / H) * (e % H) * (F::N / L) * step);
     off += (NV - 1) * H;
     L = H;
   }

@@ -2,10 +2,6 @@
 //
 //   block_params_kernel  per-block FP64 delay and fringe parameters of the F-step's
 //                        block stage (fstep.cu).
-//   window_fft_kernel    window, sideband flip, real FFT of 2M samples, channel
-//                        selection (delay_correction.cc:57-75), for the longest transforms;
-//                        up to 4096 points in window_fft.cu.
-// These FFT stages are the register-resident radix-16 transforms of fft_reg.cuh.
 //   bitstat_kernel       per-code sample counts with cal-diode on/off split, from
 //                        popcounts (bit_statistics.cc:36-47, bit2float_worker.cc:341-346).
 //   pulsar_bins_kernel / xcorr_f32_kernel  bin per (FFT, channel) in FP64 and binned
@@ -15,7 +11,6 @@
 #include <cstdio>
 
 #include "device.cuh"
-#include "fft_reg.cuh"
 #include "kernels.hpp"
 
 namespace sfxc {
@@ -134,357 +129,6 @@ __global__ void extract_kernel(const uint8_t *__restrict__ in, int64_t nout, int
   const int sb = blockIdx.y;
   if (ob >= nout) return;
   out[(int64_t)sb * nout + ob] = extract_byte(in + ob * (8 / fan_out) * N, N, bits, fan_out, tracks + sb * fan_out);
-}
-
-// ------------------------------------------------------------------------
-// F-step, stage 2: windowed real FFT of rot = 2N samples per output row as an
-// N-point complex FFT (N = 2^LOGN) of (x[2e], x[2e+1]) by T = N/16 threads,
-// then the real-FFT split and the channel selection.  For the tensor-core
-// layout ([row][channel][32 stream slots] x 8 B) one thread writes up to four
-// streams of a channel as one contiguous piece (a whole 32-byte sector for
-// four streams).
-
-// FP16 hi = fp16(s x), lo = fp16(s x - hi) of a complex value (packed
-// conversions); SCALE false: x already carries the scale s.
-template <bool SCALE>
-__device__ __forceinline__ uint2 tc_split(float2 f, float tc_scale) {
-  const float2 sv = SCALE ? make_float2(f.x * tc_scale, f.y * tc_scale) : f;
-  const __half2 h = __float22half2_rn(sv);
-  const float2 hb = __half22float2(h);
-  const __half2 l = __float22half2_rn(make_float2(sv.x - hb.x, sv.y - hb.y));
-  return make_uint2(*reinterpret_cast<const unsigned *>(&h), *reinterpret_cast<const unsigned *>(&l));
-}
-
-// Channel i of one transform Z (natural order, padded): the real-FFT split
-// for output bin q = output_offset + i - temp_fft_offset (zero outside 0..N).
-// HALF: the split's factor 1/2 applied here; else the transform's input
-// carried it (the shared window is scaled by 1/2, which is exact).
-template <int N, bool HALF>
-__device__ __forceinline__ float2 real_bin(const float2 *Z, const float2 *__restrict__ tw_rot, int q) {
-  if (q < 0 || q > N) return make_float2(0.f, 0.f);
-  const float2 zk = Z[padi(q & (N - 1))];
-  const float2 zc = Z[padi((N - q) & (N - 1))];
-  constexpr float h = HALF ? 0.5f : 1.0f;
-  const float er = h * (zk.x + zc.x), ei = h * (zk.y - zc.y);
-  const float orr = h * (zk.y + zc.y), oi = -h * (zk.x - zc.x);
-  const float2 w = __ldg(tw_rot + q);  // q <= N < rot
-  return make_float2(er + (orr * w.x - oi * w.y), ei + (orr * w.y + oi * w.x));
-}
-
-// Bins q and N - q of one transform together (0 <= q <= N/2): both read
-// Z[q] and Z[N - q], and with E, O the even and odd parts and w = tw_rot[q],
-// X[q] = E + O w and X[N - q] = conj(E - O w) (tw_rot[N - q] = -conj w).
-template <int N, bool HALF>
-__device__ __forceinline__ void real_bin_pair(const float2 *Z, float2 w, int q, float2 &xq, float2 &xnq) {
-  const float2 zk = Z[padi(q & (N - 1))];
-  const float2 zc = Z[padi((N - q) & (N - 1))];
-  constexpr float h = HALF ? 0.5f : 1.0f;
-  const float er = h * (zk.x + zc.x), ei = h * (zk.y - zc.y);
-  const float orr = h * (zk.y + zc.y), oi = -h * (zk.x - zc.x);
-  const float owr = orr * w.x - oi * w.y, owi = orr * w.y + oi * w.x;
-  xq = make_float2(er + owr, ei + owi);
-  xnq = make_float2(er - owr, owi - ei);
-}
-
-// First-pass inputs, in two steps so that the loads of the next row can be in
-// flight while the current row is written out: raw samples v[qq] = (x[2e],
-// x[2e+1]) of complex element e = t + qq T (zero from nper on, or when !ok),
-// then the window and, for a sideband flip, the negated odd samples.
-// FULL: nper = 2N (every window but NONE), no per-element bounds.
-template <int T, bool FULL>
-__device__ __forceinline__ void window_raw(float2 (&v)[16], int t, bool ok, int nper, const float *ts) {
-  if constexpr (FULL) {
-    if (ok) {
-#pragma unroll
-      for (int qq = 0; qq < 16; qq++) v[qq] = *reinterpret_cast<const float2 *>(ts + 2 * (t + qq * T));
-    } else {
-#pragma unroll
-      for (int qq = 0; qq < 16; qq++) v[qq] = make_float2(0.f, 0.f);
-    }
-  } else {
-#pragma unroll
-    for (int qq = 0; qq < 16; qq++) {
-      const int i = 2 * (t + qq * T);
-      float2 x = make_float2(0.f, 0.f);
-      if (ok && i + 1 < nper)
-        x = *reinterpret_cast<const float2 *>(ts + i);
-      else if (ok && i < nper)
-        x.x = ts[i];
-      v[qq] = x;
-    }
-  }
-}
-// The window is in shared memory (WSMEM) or read through the read-only cache.
-// FULL as for window_raw; FLIP: negate the odd samples.
-template <int T, bool WSMEM, bool FULL, bool FLIP>
-__device__ __forceinline__ void window_apply(float2 (&v)[16], int t, int nper, const float *window) {
-  if constexpr (FULL) {
-#pragma unroll
-    for (int qq = 0; qq < 16; qq++) {
-      const int i = 2 * (t + qq * T);
-      const float2 w = WSMEM ? *reinterpret_cast<const float2 *>(window + i)
-                             : __ldg(reinterpret_cast<const float2 *>(window + i));
-      v[qq] = make_float2(v[qq].x * w.x, FLIP ? -(v[qq].y * w.y) : v[qq].y * w.y);
-    }
-  } else {
-    const float sgn = FLIP ? -1.0f : 1.0f;
-#pragma unroll
-    for (int qq = 0; qq < 16; qq++) {
-      const int i = 2 * (t + qq * T);
-      if (i + 1 < nper) {
-        const float2 w = WSMEM ? *reinterpret_cast<const float2 *>(window + i)
-                               : __ldg(reinterpret_cast<const float2 *>(window + i));
-        v[qq] = make_float2(v[qq].x * w.x, sgn * (v[qq].y * w.y));
-      } else if (i < nper) {
-        v[qq] = make_float2(v[qq].x * (WSMEM ? window[i] : __ldg(window + i)), 0.f);
-      }
-    }
-  }
-}
-
-// Output row `row` of the NV <= NS streams of a CTA, whose transforms are at
-// Z + j * BUF; each goes to its slot in the spectra layout.  sinfo[j] =
-// (channel shift output_offset - temp_fft_offset, slot), staged once per CTA.
-// `fast`: four (or NS) streams with no shift in consecutive slots from a
-// multiple of four, M == N.  Threads tid = 0..nthr-1 share the channels 0..M;
-// bins q and N - q come together, so the N/2 + 1 pairs spread evenly (bin N/2
-// goes to the last threads on its own).  SCALE: the window was not the
-// pre-scaled shared copy, so the split's 1/2 and the tensor-core scale are
-// applied here.
-template <int N, int NS, int OUT_TC, bool SCALE>
-__device__ __forceinline__ void store_row(const float2 *Z, int BUF, const int2 *sinfo, int NV, bool fast, int row,
-                                          int nrows_total, int M, int kpad, const float2 *__restrict__ tw_rot,
-                                          void *__restrict__ spec_out, float tc_scale, int tid, int nthr) {
-  constexpr int S = OUT_TC;  // slots of the tensor-core layout (0: FP32 layout)
-  static_assert(NS <= 4, "at most four streams per CTA");
-  if constexpr (OUT_TC != 0) {
-    constexpr int W = NS;  // streams per store
-    uint2 *dst = reinterpret_cast<uint2 *>(spec_out);
-    if (fast) {
-      auto put = [](uint2 *p, const uint2 (&o)[W]) {
-        if constexpr (W == 1) {
-          *p = o[0];
-        } else if constexpr (W == 2) {
-          *reinterpret_cast<uint4 *>(p) = make_uint4(o[0].x, o[0].y, o[1].x, o[1].y);
-        } else if constexpr (W == 4) {
-          asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(o[0].x), "r"(o[0].y),
-                       "r"(o[1].x), "r"(o[1].y), "r"(o[2].x), "r"(o[2].y), "r"(o[3].x), "r"(o[3].y)
-                       : "memory");
-        } else {
-#pragma unroll
-          for (int j = 0; j < W; j++) p[j] = o[j];
-        }
-      };
-      const int s0 = sinfo[0].y;
-      uint2 *drow = dst + tc_index(row, kpad, 0, s0, S);  // channel i at drow + (i >> 2) * 4S + (i & 3) * 4
-      const int gs = 4 * S;
-      for (int i = tid; i < N / 2; i += nthr) {
-        const float2 w = __ldg(tw_rot + i);
-        uint2 a[W], b[W];
-#pragma unroll
-        for (int j = 0; j < W; j++) {
-          float2 xq, xnq;
-          real_bin_pair<N, SCALE>(Z + j * BUF, w, i, xq, xnq);
-          a[j] = tc_split<SCALE>(xq, tc_scale);
-          b[j] = tc_split<SCALE>(xnq, tc_scale);
-        }
-        put(drow + (i >> 2) * gs + (i & 3) * 4, a);
-        put(drow + ((N - i) >> 2) * gs + ((N - i) & 3) * 4, b);
-      }
-      if (tid >= nthr - W) {  // bin N/2, one stream per thread
-        const int j = tid - (nthr - W);
-        float2 xq, xnq;
-        real_bin_pair<N, SCALE>(Z + j * BUF, __ldg(tw_rot + N / 2), N / 2, xq, xnq);
-        dst[tc_index(row, kpad, N / 2, s0 + j, S)] = tc_split<SCALE>(xq, tc_scale);
-      }
-      return;
-    }
-    // shifted channels or scattered slots: one 8-byte store per stream and channel
-    for (int i = tid; i <= M; i += nthr)
-#pragma unroll
-      for (int j = 0; j < NS; j++)
-        if (j < NV)
-          dst[tc_index(row, kpad, i, sinfo[j].y, S)] =
-              tc_split<SCALE>(real_bin<N, SCALE>(Z + j * BUF, tw_rot, sinfo[j].x + i), tc_scale);
-  } else {
-#pragma unroll 1
-    for (int j = 0; j < NV; j++) {
-      const int shift = sinfo[j].x;
-      float2 *dst = reinterpret_cast<float2 *>(spec_out) + ((int64_t)sinfo[j].y * nrows_total + row) * kpad;
-      if (shift == 0 && M == N) {
-        for (int i = tid; i < N / 2; i += nthr) {
-          float2 xq, xnq;
-          real_bin_pair<N, SCALE>(Z + j * BUF, __ldg(tw_rot + i), i, xq, xnq);
-          dst[i] = xq;
-          dst[N - i] = xnq;
-        }
-        if (tid == nthr - 1 - j) {
-          float2 xq, xnq;
-          real_bin_pair<N, SCALE>(Z + j * BUF, __ldg(tw_rot + N / 2), N / 2, xq, xnq);
-          dst[N / 2] = xq;
-        }
-      } else {
-        for (int i = tid; i <= M; i += nthr) dst[i] = real_bin<N, SCALE>(Z + j * BUF, tw_rot, shift + i);
-      }
-    }
-  }
-}
-
-// Stage 2 as its own kernel, reading the fringe-stopped samples from s.ts:
-// a CTA of SPC x RPC groups of T threads transforms SPC streams x RPC rows per
-// step and steps through a run of rows; the next step's samples are loaded
-// into the FFT registers before the current step is written out, so those
-// HBM loads overlap the output stores.
-template <int LOGN, int SPCMAX = 4>
-struct WinShape {
-  static constexpr int N = 1 << LOGN, T = N / 16;
-  static constexpr int SPC = T * SPCMAX <= 1024 ? SPCMAX : 1024 / T;  // streams per CTA
-  static constexpr int RPC = T < 256 ? 256 / T : 1;                   // rows per step
-  static constexpr int THREADS = SPC * RPC * T;
-  static constexpr int BUF = N + N / 16;  // padded FFT buffer (float2) of one group
-  static constexpr size_t FFT_SMEM = (size_t)SPC * RPC * BUF * sizeof(float2);
-  // pass-twiddle table of the first eight twiddles per entry (17 KB at
-  // N = 4096): the shared memory still fits the same L1 carve-out as the
-  // 4-twiddle table, with four fewer complex products per pass (3 % faster);
-  // a 15-twiddle table measured 5 % slower than the 4-twiddle one, taking L1
-  // capacity from the twice-read input rows
-  static constexpr int TWK = 8;
-  static constexpr size_t PTB = pass_table_bytes<LOGN, TWK>();
-  // the window (up to rot = 2N floats) joins the shared tables when it fits
-  static constexpr bool WSMEM = FFT_SMEM + PTB + 8 * N <= 227 * 1024;
-  static constexpr size_t SMEM = FFT_SMEM + PTB + (WSMEM ? 8 * N : 0);
-  static_assert(THREADS <= 1024, "at most 1024 threads");
-};
-
-// OUT_TC: 0 writes the FP32 layout, 32 or 64 the tensor-core layout with that many slots
-template <int LOGN, int OUT_TC, int SPCMAX>
-__global__ void __launch_bounds__(WinShape<LOGN, SPCMAX>::THREADS, 1024 / WinShape<LOGN, SPCMAX>::THREADS)
-    window_fft_kernel(
-    const StreamDev *__restrict__ streams, int nstreams, int row0, int nrows, int nrows_total, int steps_per_cta,
-    const float *__restrict__ window, const float2 *__restrict__ tw_rot, int nper, int M, int kpad,
-    void *__restrict__ spec_out, float tc_scale) {
-  using S = WinShape<LOGN, SPCMAX>;
-  constexpr int N = S::N, T = S::T, SPC = S::SPC, RPC = S::RPC;
-  extern __shared__ __align__(16) float2 dsm[];
-  const int t = threadIdx.x % T, g = threadIdx.x / T;
-  const int nsg = (nstreams + SPC - 1) / SPC;
-  const int sg = blockIdx.x % nsg;  // stream group fastest
-  const int nsteps = (nrows + RPC - 1) / RPC;
-  const int k0 = (blockIdx.x / nsg) * steps_per_cta, k1 = min(nsteps, k0 + steps_per_cta);
-  const int stream = sg * SPC + g % SPC;
-  const bool sok = stream < nstreams;
-  const StreamDev &s = streams[sok ? stream : 0];
-  const bool flip = s.flip != 0;
-  // every window but NONE covers the whole transform input: no bounds per element
-  const bool full = nper == 2 * N;
-  auto row_of = [&](int k) { return k * RPC + g / SPC; };
-  auto load_row = [&](float2(&v)[16], int k) {
-    const bool ok = sok && row_of(k) < nrows;
-    const float *src = s.ts + (int64_t)(row0 + row_of(k)) * N;
-    if (full)
-      window_raw<T, true>(v, t, ok, nper, src);
-    else
-      window_raw<T, false>(v, t, ok, nper, src);
-  };
-  float2 v[16];
-  if (k0 < k1) load_row(v, k0);
-  // shared tables behind the FFT buffers: pass twiddles, then the window
-  float2 *ptab = dsm + S::FFT_SMEM / sizeof(float2);
-  fill_pass_table<LOGN, S::TWK>(ptab, tw_rot + 2 * N, threadIdx.x, S::THREADS);
-  // the CTA's streams: channel shift and slot, and whether the whole-sector path applies
-  __shared__ int2 sinfo[SPC];
-  if (threadIdx.x < SPC) {
-    const int st = sg * SPC + threadIdx.x;
-    sinfo[threadIdx.x] = st < nstreams
-                             ? make_int2(streams[st].output_offset - streams[st].temp_fft_offset, streams[st].slot)
-                             : make_int2(0, -1);
-  }
-  // a shared window carries the tensor-core layout's power-of-two scale and
-  // the real-FFT split's factor 1/2 (both exact), so the output split needs
-  // neither multiply
-  const float *win = window;
-  if constexpr (S::WSMEM) {
-    float4 *wsm = reinterpret_cast<float4 *>(ptab + S::PTB / sizeof(float2));  // nper: a multiple of 4 (rot >= 512)
-    const float ws = (OUT_TC ? tc_scale : 1.0f) * 0.5f;
-    for (int i = threadIdx.x; i < nper / 4; i += S::THREADS) {
-      const float4 w = __ldg(reinterpret_cast<const float4 *>(window) + i);
-      wsm[i] = make_float4(w.x * ws, w.y * ws, w.z * ws, w.w * ws);
-    }
-    win = reinterpret_cast<const float *>(wsm);
-  }
-  __syncthreads();
-  const int nv = min(SPC, nstreams - sg * SPC);
-  bool fast = OUT_TC && M == N && nv == SPC && sinfo[0].y % SPC == 0;
-#pragma unroll
-  for (int j = 0; j < SPC; j++) fast = fast && sinfo[j].x == 0 && sinfo[j].y == sinfo[0].y + j;
-#pragma unroll 1
-  for (int k = k0; k < k1; k++) {
-    if (full) {
-      if (flip)
-        window_apply<T, S::WSMEM, true, true>(v, t, nper, win);
-      else
-        window_apply<T, S::WSMEM, true, false>(v, t, nper, win);
-    } else {
-      if (flip)
-        window_apply<T, S::WSMEM, false, true>(v, t, nper, win);
-      else
-        window_apply<T, S::WSMEM, false, false>(v, t, nper, win);
-    }
-    // tw_rot holds exp(-2 pi i m / rot) for m < rot, followed by exp(-2 pi i m / N) for m < N.
-    // Each group's transform synchronises only its own T threads (named
-    // barrier 1 + g) when the groups are whole warps and few enough.
-    // FP32 layout: each group writes its own stream's row (whole lines), so
-    // the groups synchronise only themselves and run out of step with each
-    // other (18 % faster at 4096 channels than the CTA-wide barriers the
-    // tensor-core layout's shared 32-byte pieces need)
-    constexpr bool kIndep = OUT_TC == 0 && T >= 32 && S::THREADS / T <= 15;
-    if constexpr (kIndep) {
-      const GroupSync gs{1 + g, T};
-      fft_reg<-1, LOGN, true, S::TWK>(v, dsm + g * S::BUF, t, tw_rot + 2 * N, ptab, gs);
-      gs();
-      if (k + 1 < k1) load_row(v, k + 1);
-      const int j = g % SPC, row = row_of(k);
-      if (j < nv && row < nrows) {
-        const float2 *Z = dsm + g * S::BUF;
-        const int shift = sinfo[j].x;
-        float2 *dst = reinterpret_cast<float2 *>(spec_out) + ((int64_t)sinfo[j].y * nrows_total + row0 + row) * kpad;
-        if (shift == 0 && M == N) {
-          for (int i = t; i < N / 2; i += T) {
-            float2 xq, xnq;
-            real_bin_pair<N, !S::WSMEM>(Z, __ldg(tw_rot + i), i, xq, xnq);
-            dst[i] = xq;
-            dst[N - i] = xnq;
-          }
-          if (t == T - 1) {
-            float2 xq, xnq;
-            real_bin_pair<N, !S::WSMEM>(Z, __ldg(tw_rot + N / 2), N / 2, xq, xnq);
-            dst[N / 2] = xq;
-          }
-        } else {
-          for (int i = t; i <= M; i += T) dst[i] = real_bin<N, !S::WSMEM>(Z, tw_rot, shift + i);
-        }
-      }
-      gs();  // the next step's transform rewrites the group's buffer
-      continue;
-    }
-    if constexpr (T >= 32 && S::THREADS / T <= 15) {
-      fft_reg<-1, LOGN, true, S::TWK>(v, dsm + g * S::BUF, t, tw_rot + 2 * N, ptab, GroupSync{1 + g, T});
-      __syncthreads();  // the stores read every group's transform
-    } else {
-      fft_reg<-1, LOGN, true, S::TWK>(v, dsm + g * S::BUF, t, tw_rot + 2 * N, ptab, BlockSync());
-    }
-    if (k + 1 < k1) load_row(v, k + 1);  // hop = rot / 2
-#pragma unroll 1
-    for (int r = 0; r < RPC; r++) {
-      const int row = k * RPC + r;
-      if (row >= nrows) break;
-      store_row<N, SPC, OUT_TC, !S::WSMEM>(dsm + r * SPC * S::BUF, S::BUF, sinfo, nv, fast, row0 + row, nrows_total,
-                                           M, kpad, tw_rot, spec_out, tc_scale, threadIdx.x, S::THREADS);
-    }
-    // the next step's FFT rewrites the buffers (placing this barrier inside
-    // that FFT, after its first radix-16 pass, measured 1.7 % slower)
-    __syncthreads();
-  }
 }
 
 // ------------------------------------------------------------------------
@@ -1084,64 +728,6 @@ void launch_phasecal(const uint8_t *data, const PcalRun *runs, int nruns, int pb
     else
       phasecal_kernel<1><<<grid, 256, 0, st>>>(data, runs + r0, pb, acc);
   }
-}
-
-template <int LOGN, int OUT_TC, int SPCMAX>
-static void window_fft_launch_spc(const StreamDev *d_streams, int nstreams, int row0, int nrows, int nrows_total,
-                                  const float *window, const float2 *tw_rot, int nper, int M, int kpad, void *spec,
-                                  float tc_scale, cudaStream_t st, int waves) {
-  using S = WinShape<LOGN, SPCMAX>;
-  const int nsg = (nstreams + S::SPC - 1) / S::SPC, nsteps = (nrows + S::RPC - 1) / S::RPC;
-  // runs of steps so that the CTAs fill two waves by default (three or four
-  // waves measured 1 % slower on the 32-stream, 4096-channel job); the
-  // autotuner may pick another count per shape
-  const int per_sm = 1024 / S::THREADS;
-  const int runs = std::max(1, std::min(nsteps, (waves > 0 ? waves : 2) * per_sm * sm_count() / nsg));
-  const int steps_per_cta = (nsteps + runs - 1) / runs;
-  const unsigned grid = (unsigned)(nsg * ((nsteps + steps_per_cta - 1) / steps_per_cta));
-  auto kern = window_fft_kernel<LOGN, OUT_TC, SPCMAX>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
-  kern<<<grid, S::THREADS, S::SMEM, st>>>(d_streams, nstreams, row0, nrows, nrows_total, steps_per_cta, window, tw_rot,
-                                          nper, M, kpad, spec, tc_scale);
-}
-
-template <int LOGN, int OUT_TC>
-static void window_fft_launch(const StreamDev *d_streams, int nstreams, int row0, int nrows, int nrows_total,
-                              const float *window, const float2 *tw_rot, int nper, int M, int kpad, void *spec,
-                              float tc_scale, cudaStream_t st, int waves) {
-  // four streams per CTA: a whole 32-byte sector per channel in the TC layout
-  // (two streams per CTA, two CTAs per SM, measured 20 % slower; each group
-  // writing its own stream's 8-byte pieces, without the CTA-wide barriers,
-  // 74 % slower)
-  window_fft_launch_spc<LOGN, OUT_TC, 4>(d_streams, nstreams, row0, nrows, nrows_total, window, tw_rot, nper, M, kpad,
-                                         spec, tc_scale, st, waves);
-}
-
-#define SFXC_LOGN_SWITCH(logn, CALL) \
-  switch (logn) {                    \
-    case 13: CALL(13); break;        \
-    case 14: CALL(14); break;        \
-    default: break; /* sizes outside 2^9..2^15 samples are rejected by set_parameters */ \
-  }
-
-void launch_window_fft(const StreamDev *d_streams, int nstreams, int row0, int nrows, int nrows_total,
-                       const float *window, const float2 *tw_rot, int rot, int nper, int M, int kpad, void *spec,
-                       int tc_slots, float tc_scale, int *err, cudaStream_t st, int waves) {
-  if (launch_window_pack(d_streams, nstreams, row0, nrows, nrows_total, window, tw_rot, rot, nper, M, kpad, spec,
-                         tc_slots, tc_scale, err, st, waves))
-    return;
-  const int logn = 30 - __builtin_clz((unsigned)rot);  // log2(rot / 2)
-#define SFXC_WIN(L)                                                                                            \
-  (tc_slots == kTcSlots                                                                                         \
-       ? window_fft_launch<L, kTcSlots>(d_streams, nstreams, row0, nrows, nrows_total, window, tw_rot, nper, M,  \
-                                        kpad, spec, tc_scale, st, waves)                                      \
-   : tc_slots == kTcSlotsWide                                                                                    \
-       ? window_fft_launch<L, kTcSlotsWide>(d_streams, nstreams, row0, nrows, nrows_total, window, tw_rot, nper, \
-                                            M, kpad, spec, tc_scale, st, waves)                               \
-       : window_fft_launch<L, 0>(d_streams, nstreams, row0, nrows, nrows_total, window, tw_rot, nper, M, kpad,    \
-                                 spec, tc_scale, st, waves))
-  SFXC_LOGN_SWITCH(logn, SFXC_WIN)
-#undef SFXC_WIN
 }
 
 void launch_bitstat(const StreamDev *d_streams, const int4 *d_items, int nitems, cudaStream_t st) {

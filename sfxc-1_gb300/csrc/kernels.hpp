@@ -27,9 +27,6 @@ void launch_extract(const uint8_t *in, int64_t nout, int N, int bits, int nsub, 
 void launch_window_fft(const StreamDev *d_streams, int nstreams, int row0, int nrows, int nrows_total,
                        const float *window, const float2 *tw_rot, int rot, int nper, int M, int kpad, void *spec,
                        int tc_slots, float tc_scale, int *err, cudaStream_t st, int waves = 0);
-bool launch_window_pack(const StreamDev *d_streams, int nstreams, int row0, int nrows, int nrows_total,
-                        const float *window, const float2 *tw_rot, int rot, int nper, int M, int kpad, void *spec,
-                        int tc_slots, float tc_scale, int *err, cudaStream_t st, int waves);
 int sm_count();
 void launch_bitstat(const StreamDev *d_streams, const int4 *d_items, int nitems, cudaStream_t st);
 // FP32 X-step without binning (xcorr_f32.cu)

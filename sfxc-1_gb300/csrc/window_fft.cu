@@ -25,6 +25,11 @@ namespace {
 // NV = 16 (from 2048 points): a row's samples come by bulk copy into the
 // transform buffers while the previous row is split and written.  NV = 8
 // (up to 1024 points): many small groups, which hide each other's loads.
+// 8192 points (LONG): one packed pair fills the shared memory, so a CTA takes
+// two streams (16-byte pieces) and reads the window through the cache: the
+// streams of 8192 points of a 40-stream job, 976 rows of 4096 channels, 1.07 ->
+// 0.78 ms against one group of threads per stream.  16384 points:
+// window_long_kernel.
 //
 // What bounds it: 40.7 instructions per point (73.5 with scalar FP32 and the
 // split through shared memory) and 59 bytes of shared-memory and L1 traffic
@@ -45,12 +50,13 @@ struct PackWin {
   static constexpr bool BULK = NV == 16;
   using F = PackShape<LOGN, NV>;
   static constexpr int N = F::N, T = F::T;
-  static constexpr int S = OUT_TC || !BULK ? 2 : 1, NS = 2 * S;
+  static constexpr bool LONG = LOGN == 13;
+  static constexpr int S = (OUT_TC && !LONG) || !BULK ? 2 : 1, NS = 2 * S;
   static constexpr int THREADS = BULK && S == 2 ? 256 : 512;
   static_assert(T >= 32 && T <= THREADS, "whole warps");
   static constexpr int GROUPS = THREADS / T;
   static constexpr int BUF = S * F::ELEMS;  // one group's buffer, float4
-  static constexpr size_t SMEM = (size_t)GROUPS * BUF * 16 + ((size_t)F::tw_len() + N + N / 2 + 1) * 8;
+  static constexpr size_t SMEM = (size_t)GROUPS * BUF * 16 + ((size_t)F::tw_len() + (LONG ? 0 : N) + N / 2 + 1) * 8;
 };
 
 // FP16 hi and lo parts of both lanes of a complex pair (packed conversions)
@@ -93,11 +99,12 @@ __global__ void __launch_bounds__(PackWin<LOGN, OUT_TC>::THREADS, 1)
 
   float4 *buf = psm + g * W::BUF;
   float2 *tab = reinterpret_cast<float2 *>(psm + GROUPS * W::BUF);
-  float2 *wsm = tab + F::tw_len();  // window, N float2
-  float2 *twr = wsm + N;            // exp(-2 pi i q / 2N), q <= N/2
+  float2 *wsm = tab + F::tw_len();           // window, N float2
+  float2 *twr = wsm + (W::LONG ? 0 : N);     // exp(-2 pi i q / 2N), q <= N/2
   fill_pack_table<LOGN, NV>(tab, tw_rot + 2 * N, threadIdx.x, W::THREADS);
-  {  // the window carries the tensor-core layout's power-of-two scale and the split's 1/2 (both exact)
-    const float ws = (OUT_TC ? tc_scale : 1.0f) * 0.5f;
+  // the window carries the tensor-core layout's power-of-two scale and the split's 1/2 (both exact)
+  const float ws = (OUT_TC ? tc_scale : 1.0f) * 0.5f;
+  if (!W::LONG) {
     for (int i = threadIdx.x; i < N; i += W::THREADS) {
       const float2 w = __ldg(reinterpret_cast<const float2 *>(window) + i);
       wsm[i] = make_float2(w.x * ws, w.y * ws);
@@ -188,7 +195,13 @@ __global__ void __launch_bounds__(PackWin<LOGN, OUT_TC>::THREADS, 1)
   auto windowed = [&](cpair(&v)[NV], const float2(&x)[2][NV], int s) {
 #pragma unroll
     for (int q = 0; q < NV; q++) {
-      const float2 w = wsm[t + q * T];
+      float2 w;
+      if constexpr (W::LONG) {
+        w = __ldg(reinterpret_cast<const float2 *>(window) + t + q * T);
+        w = make_float2(w.x * ws, w.y * ws);
+      } else {
+        w = wsm[t + q * T];
+      }
       v[q].re = make_float2(x[0][q].x * w.x, x[1][q].x * w.x);
       v[q].im = make_float2(x[0][q].y * w.y, x[1][q].y * w.y);
     }
@@ -292,6 +305,8 @@ __global__ void __launch_bounds__(PackWin<LOGN, OUT_TC>::THREADS, 1)
         if constexpr (OUT_TC == 0) {
 #pragma unroll
           for (int j = 0; j < NS; j++) trow[off + j * fstride] = o[j];
+        } else if constexpr (NS == 2) {
+          *reinterpret_cast<uint4 *>(trow + off) = make_uint4(o[0].x, o[0].y, o[1].x, o[1].y);
         } else {
           asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(trow + off), "r"(o[0].x), "r"(o[0].y),
                        "r"(o[1].x), "r"(o[1].y), "r"(o[NS - 2].x), "r"(o[NS - 2].y), "r"(o[NS - 1].x),
@@ -393,32 +408,242 @@ void pack_launch(const StreamDev *d_streams, int nstreams, int row0, int nrows, 
                                           nper, M, kpad, spec, tc_scale, err);
 }
 
+// 16384 points: one stream of a row fills the shared memory, so the two packed
+// lanes are its transform's even and odd points, z[2n] and z[2n+1], in the
+// 8192-point passes; with P[k] = (A, B) their transforms, Z[k] = A + W^k B and
+// Z[k + 8192] = A - W^k B (W = exp(-2 pi i / 16384)).  The thread that holds
+// P[k] gets P[8192 - k] from its partner, and the four bins of Z that come of
+// them, k, 16384 - k, 8192 - k and 8192 + k, are two pairs of the real split,
+// which again fill the two lanes.
+//
+// Bound: in the tensor-core layout the 8-byte pieces of one stream (a partial
+// sector costs the L2 as much as a whole one); without them the chain of five
+// passes of 16 warps in step.  24 streams, 0.5 s of 64 MS/s: tensor-core layout
+// 5.53 -> 5.18 ms (5.49 with the whole window loaded after the samples have
+// landed), FP32 layout 3.55 -> 3.63 ms, against one scalar transform of 1024
+// threads.
+constexpr int kLongN = 16384;
+struct LongWin {
+  using F = PackShape<13, 16>;
+  static constexpr int N = F::N, T = F::T, THREADS = T;
+  static constexpr size_t SMEM = (size_t)F::ELEMS * 16 + ((size_t)F::tw_len() + N / 2 + 1) * 8;
+};
+
+template <int OUT_TC>
+__global__ void __launch_bounds__(LongWin::THREADS, 1)
+    window_long_kernel(const StreamDev *__restrict__ streams, int nstreams, int row0, int nrows, int nrows_total,
+                       int rows_per_group, const float *__restrict__ window, const float2 *__restrict__ tw_rot,
+                       int nper, int M, int kpad, void *__restrict__ spec_out, float tc_scale, int *__restrict__ err) {
+  using F = LongWin::F;
+  constexpr int N = LongWin::N, T = LongWin::T, NV = 16;
+  extern __shared__ __align__(16) float4 psm[];
+  const int t = threadIdx.x, lane = t & 31;
+  const StreamDev &sd = streams[blockIdx.x % nstreams];  // stream fastest
+  const int k0 = (blockIdx.x / nstreams) * rows_per_group, k1 = min(nrows, k0 + rows_per_group);
+  const bool full = nper == 2 * kLongN;
+
+  float4 *buf = psm;
+  float2 *tab = reinterpret_cast<float2 *>(psm + F::ELEMS);
+  float2 *twr = tab + F::tw_len();  // exp(-2 pi i q / 32768), q <= 4096
+  fill_pack_table<13, NV>(tab, tw_rot + 2 * kLongN, t, T, 2);
+  for (int i = t; i <= N / 2; i += T) twr[i] = __ldg(tw_rot + i);
+  const float ws = (OUT_TC ? tc_scale : 1.0f) * 0.5f;
+  __shared__ uint64_t bar;
+  if (t == 0) {
+    tc::mbar_init(&bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  const float *src = sd.ts + (int64_t)row0 * kLongN;
+  const int shift = sd.output_offset - sd.temp_fft_offset, slot = sd.slot;
+  // window scale of the even and of the odd samples (a stream in the other sideband has these negated)
+  const float wse = ws, wso = sd.flip != 0 ? -ws : ws;
+
+  const int wl = t & 15, ww = t >> 5;
+  const int tl = (t & 16) == 0 ? 16 * ww + wl : (ww == 0 && wl == 0 ? T / 2 : T - 16 * ww - wl);
+  const int partner = tl == 0 || tl == T / 2 ? lane : lane ^ 16;
+
+  const uint32_t row_bytes = (uint32_t)nper * 4;
+  int lost = -1;  // the row whose copy did not arrive in time: reported, no further copies
+  auto issue = [&](int k) {
+    if (t != 0 || k >= k1 || lost >= 0) return;
+    const float *p = src + k * (int64_t)kLongN;
+    tc::mbar_expect_tx(&bar, row_bytes);
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     tc::smem_u32(buf)),
+                 "l"(p), "r"(row_bytes), "r"(tc::smem_u32(&bar))
+                 : "memory");
+    if (k + 1 < k1)
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p + nper), "r"(4 * kLongN) : "memory");
+  };
+  // offsets of the thread's channels tl + T m, N - tl - T m, N + tl + T m and
+  // 2 N - tl - T m of a row at m = 0
+  int ch[4], off[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    ch[i] = (i & 1 ? -tl : tl) + (i == 0 ? 0 : i == 3 ? 2 * N : N) - shift;
+    off[i] = OUT_TC ? (int)tc_index(0, kpad, ch[i], slot, OUT_TC) : ch[i];
+  }
+  constexpr int STEP = OUT_TC ? T * OUT_TC : T;
+
+  issue(k0);
+#pragma unroll 1
+  for (int k = k0; k < k1; k++) {
+    {
+      cpair v[1][NV];
+      float4 w0[NV / 2];  // the window of the first half, on its way while the samples land
+#pragma unroll
+      for (int q = 0; q < NV / 2; q++) w0[q] = __ldg(reinterpret_cast<const float4 *>(window) + t + q * T);
+      if (lost < 0 && !tc::mbar_wait(&bar, (uint32_t)(k - k0) & 1)) {
+        atomicExch(err, 1);
+        lost = k;
+      }
+#pragma unroll
+      for (int q = 0; q < NV; q++) {
+        if (q < NV / 2 || full) {
+          const float4 w = q < NV / 2 ? w0[q % (NV / 2)] : __ldg(reinterpret_cast<const float4 *>(window) + t + q * T);
+          const float4 x = buf[t + q * T];
+          v[0][q].re = make_float2(x.x * (w.x * wse), x.z * (w.z * wse));
+          v[0][q].im = make_float2(x.y * (w.y * wso), x.w * (w.w * wso));
+        } else {
+          v[0][q] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        }
+      }
+      dftn(v[0]);
+      pack_first<13>(v, buf, tab, t, [] { __syncthreads(); });
+    }
+    __syncthreads();
+    pack_middle<13, 1, NV, 1>(buf, tab, t);
+    __syncthreads();
+    pack_middle<13, 1, NV, 2>(buf, tab, t);
+    __syncthreads();
+    cpair z[NV];
+    pack_last<13>(z, buf, tl);
+    // once every thread has read the buffer, the next row's samples may come
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    issue(k + 1);
+    // the upper half goes to the partner; thread 0 pairs T m with T (16 - m)
+    // and has the middle, N/2 = 8 T, to itself
+    const cpair zmid = z[NV / 2];
+    if (t < 32) {
+      const cpair z0 = z[0];
+      if (tl == 0) {
+#pragma unroll
+        for (int m = NV / 2; m < NV - 1; m++) z[m] = z[m + 1];
+        z[NV - 1] = z0;
+      }
+    }
+    uint2 *trow = reinterpret_cast<uint2 *>(spec_out) +
+                  (OUT_TC ? (int64_t)(row0 + k) * kpad * OUT_TC : ((int64_t)slot * nrows_total + row0 + k) * kpad);
+    auto store = [&](int c, int o, float re, float im) {
+      if ((unsigned)c > (unsigned)M) return;
+      if constexpr (OUT_TC != 0) {
+        const __half2 h = __floats2half2_rn(re, im);
+        const float2 f = __half22float2(h);
+        const __half2 l = __floats2half2_rn(re - f.x, im - f.y);
+        trow[o] = make_uint2(*reinterpret_cast<const unsigned *>(&h), *reinterpret_cast<const unsigned *>(&l));
+      } else {
+        trow[o] = make_uint2(__float_as_uint(re), __float_as_uint(im));
+      }
+    };
+    // P[b] and P[8192 - b], w = exp(-2 pi i b / 32768), u = w^2 = W^b -> bins
+    // b, 16384 - b (first lane), 8192 - b, 8192 + b (second); the first of a
+    // lane is E + O w, the second conj(E - O w), the second lane's w -i conj(w)
+    auto bins = [&](cpair a, cpair c, float2 w, float2 u, cpair &xq, cpair &xn) {
+      const cpair A = {make_float2(a.re.x, c.re.x), make_float2(a.im.x, c.im.x)};
+      const cpair B = {make_float2(a.re.y, c.re.y), make_float2(a.im.y, c.im.y)};
+      // W^b B of the first lane, W^(8192 - b) B = -conj(W^b) B of the second
+      const float2 ux = make_float2(u.x, -u.x);
+      const cpair tw = {fma2(B.re, ux, mul2(B.im, dup2(-u.y))), fma2(B.re, dup2(u.y), mul2(B.im, ux))};
+      const cpair zk = A + tw, d = A - tw;
+      const cpair zc = {make_float2(d.re.y, d.re.x), make_float2(d.im.y, d.im.x)};
+      const float2 er = add2(zk.re, zc.re), ei = sub2(zk.im, zc.im);
+      const cpair o = {add2(zk.im, zc.im), sub2(zc.re, zk.re)};
+      const float2 wx = make_float2(w.x, -w.y), wy = make_float2(w.y, -w.x), ny = make_float2(-w.y, w.x);
+      const cpair ow = {fma2(o.re, wx, mul2(o.im, ny)), fma2(o.re, wy, mul2(o.im, wx))};
+      xq = {add2(er, ow.re), add2(ei, ow.im)};
+      xn = {sub2(er, ow.re), sub2(ow.im, ei)};
+    };
+    const float2 *w14 = tw_rot + 2 * kLongN;
+    float2 u = __ldg(w14 + tl);
+#pragma unroll
+    for (int m = 0; m < NV / 2; m++) {
+      const float2 um = u;
+      if (m + 1 < NV / 2) u = __ldg(w14 + tl + T * (m + 1));
+      const cpair zc = {shfl2(z[NV - 1 - m].re, partner), shfl2(z[NV - 1 - m].im, partner)};
+      cpair xq, xn;
+      bins(z[m], zc, twr[tl + T * m], um, xq, xn);
+      store(ch[0] + T * m, off[0] + STEP * m, xq.re.x, xq.im.x);
+      store(ch[3] - T * m, off[3] - STEP * m, xn.re.x, xn.im.x);
+      store(ch[1] - T * m, off[1] - STEP * m, xq.re.y, xq.im.y);
+      store(ch[2] + T * m, off[2] + STEP * m, xn.re.y, xn.im.y);
+    }
+    if (t < 32 && tl == 0) {  // b = 8192 - b
+      cpair xq, xn;
+      bins(zmid, zmid, twr[N / 2], __ldg(w14 + N / 2), xq, xn);
+      store(ch[0] + T * NV / 2, off[0] + STEP * NV / 2, xq.re.x, xq.im.x);
+      store(ch[3] - T * NV / 2, off[3] - STEP * NV / 2, xn.re.x, xn.im.x);
+    }
+  }
+  if (lost >= 0) tc::mbar_wait(&bar, (uint32_t)(lost - k0) & 1);  // bounded; nothing lands after the CTA has gone
+  // channels outside the stream's bins (a stream that covers part of the band)
+  if (shift >= 0 && shift + M <= kLongN) return;
+#pragma unroll 1
+  for (int r = k0; r < k1; r++)
+    for (int c = t; c <= M; c += T) {
+      if ((unsigned)(c + shift) <= (unsigned)kLongN) continue;
+      if constexpr (OUT_TC != 0)
+        reinterpret_cast<uint2 *>(spec_out)[tc_index(row0 + r, kpad, c, slot, OUT_TC)] = make_uint2(0u, 0u);
+      else
+        reinterpret_cast<float2 *>(spec_out)[((int64_t)slot * nrows_total + row0 + r) * kpad + c] =
+            make_float2(0.f, 0.f);
+    }
+}
+
+template <int OUT_TC>
+void long_launch(const StreamDev *d_streams, int nstreams, int row0, int nrows, int nrows_total, const float *window,
+                 const float2 *tw_rot, int nper, int M, int kpad, void *spec, float tc_scale, int *err, cudaStream_t st,
+                 int waves) {
+  const int ctas = std::max(1, (waves > 0 ? waves : 2) * sm_count() / nstreams);
+  const int rows_per_group = std::max(1, (nrows + ctas - 1) / ctas);
+  const unsigned grid = (unsigned)(nstreams * ((nrows + rows_per_group - 1) / rows_per_group));
+  auto kern = window_long_kernel<OUT_TC>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LongWin::SMEM);
+  kern<<<grid, LongWin::THREADS, LongWin::SMEM, st>>>(d_streams, nstreams, row0, nrows, nrows_total, rows_per_group,
+                                                      window, tw_rot, nper, M, kpad, spec, tc_scale, err);
+}
+
 }  // namespace
 
-bool launch_window_pack(const StreamDev *d_streams, int nstreams, int row0, int nrows, int nrows_total,
-                        const float *window, const float2 *tw_rot, int rot, int nper, int M, int kpad, void *spec,
-                        int tc_slots, float tc_scale, int *err, cudaStream_t st, int waves) {
-#define SFXC_PACK(L)                                                                                              \
-  case 2 << L:                                                                                                    \
-    if (tc_slots == kTcSlots)                                                                                     \
-      pack_launch<L, kTcSlots>(d_streams, nstreams, row0, nrows, nrows_total, window, tw_rot, nper, M, kpad, spec, \
-                               tc_scale, err, st, waves);                                                              \
-    else if (tc_slots == kTcSlotsWide)                                                                            \
-      pack_launch<L, kTcSlotsWide>(d_streams, nstreams, row0, nrows, nrows_total, window, tw_rot, nper, M, kpad,  \
-                                   spec, tc_scale, err, st, waves);                                                    \
-    else                                                                                                          \
-      pack_launch<L, 0>(d_streams, nstreams, row0, nrows, nrows_total, window, tw_rot, nper, M, kpad, spec,       \
-                        tc_scale, err, st, waves);                                                                     \
-    return true;
+void launch_window_fft(const StreamDev *d_streams, int nstreams, int row0, int nrows, int nrows_total,
+                       const float *window, const float2 *tw_rot, int rot, int nper, int M, int kpad, void *spec,
+                       int tc_slots, float tc_scale, int *err, cudaStream_t st, int waves) {
+#define SFXC_WINDOW(points, launch, ...)                                                                         \
+  case 2 * points:                                                                                             \
+    if (tc_slots == kTcSlots)                                                                                  \
+      launch<__VA_ARGS__ kTcSlots>(d_streams, nstreams, row0, nrows, nrows_total, window, tw_rot, nper, M, kpad,   \
+                                   spec, tc_scale, err, st, waves);                                               \
+    else if (tc_slots == kTcSlotsWide)                                                                         \
+      launch<__VA_ARGS__ kTcSlotsWide>(d_streams, nstreams, row0, nrows, nrows_total, window, tw_rot, nper, M,     \
+                                       kpad, spec, tc_scale, err, st, waves);                                     \
+    else                                                                                                       \
+      launch<__VA_ARGS__ 0>(d_streams, nstreams, row0, nrows, nrows_total, window, tw_rot, nper, M, kpad, spec,    \
+                            tc_scale, err, st, waves);                                                            \
+    break;
+#define SFXC_COMMA ,
   switch (rot) {
-    SFXC_PACK(8)
-    SFXC_PACK(9)
-    SFXC_PACK(10)
-    SFXC_PACK(11)
-    SFXC_PACK(12)
-    default: return false;
+    SFXC_WINDOW(256, pack_launch, 8 SFXC_COMMA)
+    SFXC_WINDOW(512, pack_launch, 9 SFXC_COMMA)
+    SFXC_WINDOW(1024, pack_launch, 10 SFXC_COMMA)
+    SFXC_WINDOW(2048, pack_launch, 11 SFXC_COMMA)
+    SFXC_WINDOW(4096, pack_launch, 12 SFXC_COMMA)
+    SFXC_WINDOW(8192, pack_launch, 13 SFXC_COMMA)
+    SFXC_WINDOW(16384, long_launch, )
+    default: break;  // sizes outside 2^9..2^15 samples are rejected by set_parameters
   }
-#undef SFXC_PACK
+#undef SFXC_COMMA
+#undef SFXC_WINDOW
 }
 
 }  // namespace sfxc
