@@ -537,27 +537,79 @@ __global__ void phased_kernel(const float2 *__restrict__ spec, int nrows_total, 
 // a cross baseline of centre c >= 1 first gets the amplitude and the phase
 // phi + k delta of its residual delay (FP64 angle, FP32 product, as the
 // reference's FP64 recurrence and complex<float> arithmetic).
-__global__ void pc_dump_kernel(float2 *__restrict__ acc, float2 *__restrict__ pcacc, const UvShift *__restrict__ uvp,
-                               int nstreams, int nbl, int kpad, int K, int npc) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
-  if (k >= K) return;
-  const size_t i = (size_t)b * kpad + k, cstride = (size_t)nbl * kpad;
-  const float2 x = acc[i];
-  pcacc[i] = make_float2(pcacc[i].x + x.x, pcacc[i].y + x.y);
-  for (int c = 1; c < npc; c++) {
-    float2 &p = pcacc[c * cstride + i];
-    if (b < nstreams) {
-      p = make_float2(p.x + x.x, p.y + x.y);
-    } else {
-      const UvShift u = uvp[(size_t)(c - 1) * nbl + b];
-      double sn, cs;
-      sincos(fma((double)k, u.delta, u.phi), &sn, &cs);
-      const float amp = (float)u.amp, cf = (float)cs, sf = (float)sn;
-      const float xr = amp * x.x, xi = amp * x.y;
-      p = make_float2(p.x + (xr * cf - xi * sf), p.y + (xr * sf + xi * cf));
+//
+// A thread takes kPcChans channels, kPcThreads apart.  Its first channel's
+// factor is the FP64 product of two table entries (16 runs of 8 channels, 8
+// channels of a run), the next ones follow by an FP64 rotation of kPcThreads
+// steps; the CTA computes the tables' sines and cosines, 25 a centre, five
+// centres at once.  At most 16 products of rounding 1e-16 each, far below the
+// FP32 product.  Bound by the FP64 pipe: 16 centres, 120 cross baselines, 2048
+// channels 217 -> 120 us a sub-integration (a sine and cosine per channel
+// before; one per thread and centre 150).
+constexpr int kPcThreads = 128, kPcChans = 16, kPcTab = 25, kPcBatch = kPcThreads / kPcTab;
+__global__ void __launch_bounds__(kPcThreads) pc_dump_kernel(float2 *__restrict__ acc, float2 *__restrict__ pcacc,
+                                                             const UvShift *__restrict__ uvp, int nstreams, int nbl,
+                                                             int kpad, int K, int npc) {
+  // of the next centres: exp(i (phi + (first channel + 8 e) delta)), e < 16;
+  // exp(i e delta), e < 8; exp(i kPcThreads delta)
+  __shared__ double2 tab[kPcBatch][kPcTab];
+  const int t = threadIdx.x, k0 = blockIdx.x * kPcThreads * kPcChans + t, b = blockIdx.y;
+  const size_t i0 = (size_t)b * kpad + k0, cstride = (size_t)nbl * kpad;
+  const int n = k0 < K ? min(kPcChans, (K - 1 - k0) / kPcThreads + 1) : 0;
+  float2 x[kPcChans];
+#pragma unroll
+  for (int j = 0; j < kPcChans; j++) {
+    if (j >= n) break;
+    x[j] = acc[i0 + j * kPcThreads];
+  }
+#pragma unroll
+  for (int j = 0; j < kPcChans; j++) {
+    if (j >= n) break;
+    const float2 y = pcacc[i0 + j * kPcThreads];
+    pcacc[i0 + j * kPcThreads] = make_float2(y.x + x[j].x, y.y + x[j].y);
+    acc[i0 + j * kPcThreads] = make_float2(0.f, 0.f);
+  }
+  for (int c0 = 1; c0 < npc; c0 += kPcBatch) {
+    const int c1 = min(npc, c0 + kPcBatch);
+    if (b >= nstreams) {
+      __syncthreads();
+      const int tc = t / kPcTab, e = t % kPcTab;
+      if (c0 + tc < c1) {
+        const UvShift u = uvp[(size_t)(c0 + tc - 1) * nbl + b];
+        const double angle = e < 16   ? fma((double)(k0 - t + 8 * e), u.delta, u.phi)
+                             : e < 24 ? (e - 16) * u.delta
+                                      : kPcThreads * u.delta;
+        double sn, cs;
+        sincos(angle, &sn, &cs);
+        tab[tc][e] = make_double2(cs, sn);
+      }
+      __syncthreads();
+    }
+    if (n == 0) continue;
+    for (int c = c0; c < c1; c++) {
+      float2 *p = pcacc + c * cstride + i0;
+      float2 y[kPcChans];  // all on their way together
+#pragma unroll
+      for (int j = 0; j < kPcChans; j++) y[j] = j < n ? p[j * kPcThreads] : make_float2(0.f, 0.f);
+      if (b < nstreams) {
+#pragma unroll
+        for (int j = 0; j < kPcChans; j++)
+          if (j < n) p[j * kPcThreads] = make_float2(y[j].x + x[j].x, y[j].y + x[j].y);
+        continue;
+      }
+      const float amp = (float)uvp[(size_t)(c - 1) * nbl + b].amp;
+      const double2 r0 = tab[c - c0][t >> 3], r1 = tab[c - c0][16 + (t & 7)], st = tab[c - c0][24];
+      double cs = fma(r0.x, r1.x, -(r0.y * r1.y)), sn = fma(r0.x, r1.y, r0.y * r1.x);
+#pragma unroll
+      for (int j = 0; j < kPcChans; j++) {
+        const float cf = (float)cs, sf = (float)sn, xr = amp * x[j].x, xi = amp * x[j].y;
+        if (j < n) p[j * kPcThreads] = make_float2(y[j].x + (xr * cf - xi * sf), y[j].y + (xr * sf + xi * cf));
+        const double nc = fma(cs, st.x, -(sn * st.y));
+        sn = fma(cs, st.y, sn * st.x);
+        cs = nc;
+      }
     }
   }
-  acc[i] = make_float2(0.f, 0.f);
 }
 
 // ------------------------------------------------------------------------
@@ -741,7 +793,10 @@ void launch_phased(const float2 *spec, int nrows_total, int kpad, int nstreams, 
 
 void launch_pc_dump(float2 *acc, float2 *pcacc, const UvShift *uvp, int nstreams, int nbl, int kpad, int K, int npc,
                     cudaStream_t st) {
-  if (nbl > 0) pc_dump_kernel<<<dim3((K + 255) / 256, nbl), 256, 0, st>>>(acc, pcacc, uvp, nstreams, nbl, kpad, K, npc);
+  const int chans = kPcThreads * kPcChans;
+  if (nbl > 0)
+    pc_dump_kernel<<<dim3((K + chans - 1) / chans, nbl), kPcThreads, 0, st>>>(acc, pcacc, uvp, nstreams, nbl, kpad, K,
+                                                                              npc);
 }
 
 cudaError_t launch_reduce(const float2 *in, int nbl, int nout, int M, int nch, const float *mask,
