@@ -1147,16 +1147,17 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
     }
   }
   size_t ev = 0;
-  // Chunk ch's X-step runs on the third stream beside chunk ch + 1's F-step
-  // (an X-step CTA and an F-step CTA fit an SM together); chunk ch + 1's
-  // windowed FFT, which overwrites the spectra, waits for it (the phases'
+  // Chunk ch's X-step and phase-centre dump run on the third stream beside
+  // chunk ch + 1's F-step, whose CTAs take the SMs they leave; chunk ch + 1's
+  // windowed FFT, which overwrites the spectra, waits for them (the phases'
   // times then overlap: each is its own kernels' elapsed time).  Measured
-  // at 4096 channels: the FP32 X-step path 5-6 % faster overall (16- and
-  // 32-stream jobs), a batch with row-gathered tensor-core X-steps (40-stream
-  // jobs) 5 %; the TMA-fed X-step 1.3-3 % slower, whatever its CTA count
-  // (with 129 KB of shared memory it leaves room for one of the F-step's four
-  // CTAs per SM, so the F-step's time grows by about what the X-step takes),
-  // so it stays on the main stream.
+  // against the main stream: with 15 extra phase centres 5.2 against 5.7 ms, a
+  // batch with row-gathered tensor-core X-steps (40-stream jobs) 16.4 against
+  // 16.5, FP32 X-steps of 16 and 32 streams and the 40-stream job alone the
+  // same; the TMA-fed X-step 1.3-3 % slower, whatever its CTA count (with 131
+  // KB of shared memory it leaves an SM room for little of the F-step, so the
+  // F-step's time grows by about what the X-step takes), so it stays on the
+  // main stream.
   const size_t R = ranges.size();
   cudaStream_t xs = tc_tma ? st : c->st3;
   for (size_t ch = 0; ch < R; ch++) {
