@@ -14,7 +14,7 @@
 // apart, 8-row groups 256 nq bytes apart.  The M index of a component is
 // 4 * stream + {hi.re, hi.im, lo.re, lo.im}.  Only the slot quads that hold
 // streams are loaded (24 streams, 16384 channels, 0.5 s: 1.74 -> 1.45 ms).  The MMA computes
-// D = A A^T (128 x 128, FP32 accumulation in TMEM); summing the four hi/lo
+// D = A A^T (128 x 16 nq, FP32 accumulation in TMEM); summing the four hi/lo
 // combinations of a stream pair gives the compensated product, and the
 // epilogue forms
 //   Re V(a,b) = sum over re-re and im-im pairs,  Im V(a,b) = im-re minus re-im
