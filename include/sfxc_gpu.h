@@ -198,7 +198,8 @@ int sfxc_gpu_run_integration(sfxc_gpu_ctx *ctx, sfxc_output_sink sink, void *use
 /* Inspection of the last integration (for verification).  Copies stream
  * `stream`'s unpacked samples (n_blocks * fft_size_delaycor floats, the
  * output of Bit2float_worker) or its delay-corrected spectra (rows of
- * fft_size_correlation + 1 complex values, the output of Delay_correction). */
+ * fft_size_correlation + 1 complex values, the output of Delay_correction).
+ * SFXC_GPU_ESTATE when no integration with that stream has run. */
 int sfxc_gpu_copy_unpacked(sfxc_gpu_ctx *ctx, int32_t stream, float *out, size_t n_floats);
 int sfxc_gpu_copy_spectra(sfxc_gpu_ctx *ctx, int32_t stream, float *out, size_t n_floats);
 /* Pulsar bin of every FFT row and channel of the last integration (the bins

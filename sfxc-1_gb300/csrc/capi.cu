@@ -314,11 +314,14 @@ struct sfxc_gpu_ctx {
     void *spec = nullptr;
     std::vector<std::array<int, 3>> groups;
   } tune;
-  // bit-statistics counters of all streams (8 per stream) and the kernels'
-  // error flag; the pinned landing area of an integration's results holds
-  // them, then the outputs in their file layout (two readback copies)
+  // the kernels' error flag (kFlagBytes) and the bit-statistics counters of all
+  // streams (8 per stream); the pinned landing area of an integration's results
+  // holds them, then the outputs in their file layout (two readback copies)
   DevBuf hist;
+  // stream descriptors of the last integration planned, and whether the last
+  // plan's tables are on the device (the inspection calls read them)
   std::vector<StreamDev> hsd;
+  bool tables_ready = false;
   // buffers of destroyed recordings, for the next ones
   std::vector<std::unique_ptr<RecordingBuffers>> rec_spare;
 };
@@ -760,10 +763,20 @@ void write_headers(sfxc_gpu_ctx *c, const std::vector<Baseline> &bls, int32_t so
   }
 }
 
-// The kernels' error flag: behind the bit-statistics counters, cleared and
-// read back with them.
-int *device_error(sfxc_gpu_ctx *c) {
-  return c->hist.p ? reinterpret_cast<int *>(c->hist.as<uint8_t>() + c->streams.size() * 64) : nullptr;
+// The kernels' error flag: ahead of the bit-statistics counters, cleared and
+// read back with them.  Its place does not depend on the job, whose stream
+// count may already be the next integration's while hist is the last one's.
+constexpr size_t kFlagBytes = 16;
+int *device_error(sfxc_gpu_ctx *c) { return c->hist.as<int>(); }
+
+// Descriptor of a stream in the last integration, for the inspection calls.
+// Its input is wherever later pushes have moved it.
+StreamDev last_stream(const sfxc_gpu_ctx *c, int stream) {
+  if (!c->tables_ready || stream >= (int)c->hsd.size())
+    throw Error(SFXC_GPU_ESTATE, "no integration with this stream has run yet");
+  StreamDev d = c->hsd[stream];
+  d.src = c->sc[stream].src.as<uint8_t>();
+  return d;
 }
 
 // Node interval (the device search's answer) of the first block start of a
@@ -808,9 +821,10 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
   const int M = c->M, K = c->K, kpad = c->kpad, nbl = (int)c->bl.size();
   cudaStream_t st = c->st;
   // ---- host planning per stream (Bit2float_worker state machine replica)
+  c->tables_ready = false;
   c->hsd.assign(N, StreamDev{});
-  c->hist.ensure((size_t)N * 64 + 16);
-  q.memset(c->hist.p, 0, (size_t)N * 64 + 16, st);
+  c->hist.ensure(kFlagBytes + (size_t)N * 64);
+  q.memset(c->hist.p, 0, kFlagBytes + (size_t)N * 64, st);
   std::vector<int4> items;
   for (int i = 0; i < N; i++) {
     StreamCtx &s = c->sc[i];
@@ -888,7 +902,7 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
       d.output_offset = 0;
       d.temp_fft_offset = (int)(-delta * 2 * M / c->p.sample_rate);
     }
-    d.hist = c->hist.as<unsigned long long>() + (size_t)i * 8;
+    d.hist = reinterpret_cast<unsigned long long *>(c->hist.as<uint8_t>() + kFlagBytes) + (size_t)i * 8;
     d.phase_zero = std::all_of(s.sp.y[1].begin(), s.sp.y[1].end(), [](double v) { return v == 0.0; });
     d.amp_one = std::all_of(s.sp.y[2].begin(), s.sp.y[2].end(), [](double v) { return v == 1.0; });
     d.no_clock = s.sp.clock_offset == 0.0 && s.sp.clock_rate == 0.0;
@@ -1330,12 +1344,12 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
       launches += 1;
     }
   }
-  const size_t res_out = (size_t)N * 64 + 16 + kOutBase;
+  const size_t res_out = kFlagBytes + (size_t)N * 64 + kOutBase;
   uint8_t *res = static_cast<uint8_t *>(sl.results.ensure(res_out + out_bytes));
   {
     const void *histp = c->hist.p;
     q.op([=] { return cudaMemcpyAsync(res + res_out, outp, out_bytes, cudaMemcpyDeviceToHost, st); });
-    q.op([=] { return cudaMemcpyAsync(res, histp, (size_t)N * 64 + 16, cudaMemcpyDeviceToHost, st); });
+    q.op([=] { return cudaMemcpyAsync(res, histp, kFlagBytes + (size_t)N * 64, cudaMemcpyDeviceToHost, st); });
   }
   q.mark(sl.evs[ev + 1], st);
   Pending &pd = sl.pend;
@@ -1373,11 +1387,12 @@ void prepare_outputs(sfxc_gpu_ctx *c, int k, IntegrationOut &out) {
   const int launches = pd.launches;
   const std::vector<std::pair<int64_t, int64_t>> &nfl = pd.nfl;
   uint8_t *res = pd.res;
-  const unsigned long long *hist = reinterpret_cast<const unsigned long long *>(res);
-  const int *dev_err = reinterpret_cast<const int *>(res + (size_t)N * 64);
+  const int *dev_err = reinterpret_cast<const int *>(res);
+  const unsigned long long *hist = reinterpret_cast<const unsigned long long *>(res + kFlagBytes);
   cudaStream_t st = c->st;
   float t_f1 = 0, t_f2 = 0, t_x = 0;
   CK(cudaStreamSynchronize(st));
+  c->tables_ready = true;
   if (*dev_err) throw Error(SFXC_GPU_ECUDA, "a kernel timed out waiting for its copies or MMAs");
   // per chunk: F-step start and end, windowed FFT start (after the previous
   // X-step when that ran beside the F-step) and end, X-step end
@@ -1414,7 +1429,7 @@ void prepare_outputs(sfxc_gpu_ctx *c, int k, IntegrationOut &out) {
     bs.base_sample_rate = c->p.sample_rate;
   }
   // ---- output headers (integration_write per bin) and tsys records
-  uint8_t *o = res + (size_t)N * 64 + 16 + kOutBase;
+  uint8_t *o = res + kFlagBytes + (size_t)N * 64 + kOutBase;
   out.cor = o;
   if (c->phased) {
     write_headers(c, std::vector<Baseline>(nphs, Baseline{0, 0}), 0, 0, nfl, o);
@@ -1612,7 +1627,7 @@ int sfxc_gpu_copy_unpacked(sfxc_gpu_ctx *c, int32_t stream, float *out, size_t n
     const StreamCtx &s = c->sc[stream];
     const size_t need = (size_t)s.n_blocks * c->Nd;
     if (n < need) throw Error(SFXC_GPU_EINVAL, "output buffer too small");
-    StreamDev d = c->hsd[stream];
+    StreamDev d = last_stream(c, stream);
     DevBuf sd, dout;
     dout.ensure(need * sizeof(float));
     upload(sd, &d, sizeof(StreamDev), c->st);
@@ -1735,7 +1750,7 @@ int sfxc_gpu_copy_spectra(sfxc_gpu_ctx *c, int32_t stream, float *out, size_t n)
     const StreamCtx &s = c->sc[stream];
     const size_t rows = (size_t)c->nffts, K = (size_t)c->M + 1;
     if (n < rows * K * 2) throw Error(SFXC_GPU_EINVAL, "output buffer too small");
-    StreamDev d = c->hsd[stream];
+    StreamDev d = last_stream(c, stream);
     d.block0 = 0;
     d.n_blocks = s.n_blocks;
     d.spline_lo = spline_lo_for(d, s.sp.x);  // the block kernel walks the spline forward from block 0
@@ -1748,7 +1763,7 @@ int sfxc_gpu_copy_spectra(sfxc_gpu_ctx *c, int32_t stream, float *out, size_t n)
     d.bpar = bp.as<BlockPar>();
     upload(sd, &d, sizeof(StreamDev), c->st);
     int err = 0;
-    if (device_error(c)) CK(cudaMemsetAsync(device_error(c), 0, sizeof(int), c->st));
+    CK(cudaMemsetAsync(device_error(c), 0, sizeof(int), c->st));
     launch_fstep_block(sd.as<StreamDev>(), 1, s.n_blocks, c->tw256.as<float2>(), c->st);
     const int nper = c->p.window == WINDOW_NONE ? s.hop : s.rot;
     const sfxc_gpu_ctx::RotTables &t = c->rot_tables.at(s.rot);
@@ -1757,7 +1772,7 @@ int sfxc_gpu_copy_spectra(sfxc_gpu_ctx *c, int32_t stream, float *out, size_t n)
     CK(cudaGetLastError());
     CK(cudaMemcpy2DAsync(out, K * sizeof(float2), spec.p, c->kpad * sizeof(float2), K * sizeof(float2), rows,
                          cudaMemcpyDeviceToHost, c->st));
-    if (device_error(c)) CK(cudaMemcpyAsync(&err, device_error(c), sizeof(int), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(&err, device_error(c), sizeof(int), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     if (err) throw Error(SFXC_GPU_ECUDA, "a kernel timed out waiting for its copies");
     return (int)(rows * K * 2);
@@ -1827,7 +1842,7 @@ int sfxc_gpu_copy_spectra_noalloc(sfxc_gpu_ctx *c, int32_t stream, float *out, s
                                        std::to_string(kNoallocMaxSpectra) + " complex values)");
     CK(cudaSetDevice(c->device));
     unsigned char *base = noalloc_scratch(c->device);
-    StreamDev d = c->hsd[stream];
+    StreamDev d = last_stream(c, stream);
     d.block0 = 0;
     d.n_blocks = s.n_blocks;
     d.spline_lo = spline_lo_for(d, s.sp.x);  // the block kernel walks the spline forward from block 0
@@ -1840,7 +1855,7 @@ int sfxc_gpu_copy_spectra_noalloc(sfxc_gpu_ctx *c, int32_t stream, float *out, s
     // nothing is cleared; the descriptor copy is ordered on the context stream
     CK(cudaMemcpyAsync(dd, &d, sizeof(StreamDev), cudaMemcpyHostToDevice, c->st));
     int err = 0;
-    if (device_error(c)) CK(cudaMemsetAsync(device_error(c), 0, sizeof(int), c->st));
+    CK(cudaMemsetAsync(device_error(c), 0, sizeof(int), c->st));
     launch_fstep_block(dd, 1, s.n_blocks, c->tw256.as<float2>(), c->st);
     const int nper = c->p.window == WINDOW_NONE ? s.hop : s.rot;
     const sfxc_gpu_ctx::RotTables &t = c->rot_tables.at(s.rot);
@@ -1849,7 +1864,7 @@ int sfxc_gpu_copy_spectra_noalloc(sfxc_gpu_ctx *c, int32_t stream, float *out, s
     CK(cudaGetLastError());
     CK(cudaMemcpy2DAsync(out, K * sizeof(float2), spec, c->kpad * sizeof(float2), K * sizeof(float2), rows,
                          cudaMemcpyDeviceToHost, c->st));
-    if (device_error(c)) CK(cudaMemcpyAsync(&err, device_error(c), sizeof(int), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(&err, device_error(c), sizeof(int), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     if (err) throw Error(SFXC_GPU_ECUDA, "a kernel timed out waiting for its copies");
     return (int)(rows * K * 2);
