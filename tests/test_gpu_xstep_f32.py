@@ -39,3 +39,10 @@ def test_fp32_xstep_shapes(streams, rows, ref, pols):
     assert h0 == h1
     a, b = np.array(v0).astype(np.complex128), np.array(v1).astype(np.complex128)
     assert np.linalg.norm(a - b) < 2e-6 * np.linalg.norm(b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("streams,rows,ref", [(35, 40, -1), (65, 12, -1), (72, 300, 1), (100, 9, -1), (128, 5, 2)])
+def test_fp32_xstep_wide(streams, rows, ref):
+    """Parts that leave warps without a unit, steps of a single row (from 65 streams), up to 128 streams."""
+    test_fp32_xstep_shapes(streams, rows, ref, 1)
