@@ -68,7 +68,8 @@ __device__ __forceinline__ void tile_row(float2 (&v)[8][8], const float2 *xa, co
     }
 }
 
-__global__ void __launch_bounds__(256, 1) xcorr_tile8_kernel(const __grid_constant__ TileArgs a) {
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) xcorr_tile8_kernel(const __grid_constant__ TileArgs a) {
   extern __shared__ __align__(16) float2 xs[];  // kRing x [R rows][np8 streams][32 channels]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, G = a.groups;
   const int wu = warp % a.units_per_part, wg = warp / a.units_per_part;  // unit of the part, row group
@@ -229,11 +230,17 @@ struct TilePlan {
 TilePlan tile_plan(int nunits, int nstreams, int K, int nrows) {
   TilePlan p{};
   const int np8 = (nstreams + 7) / 8 * 8, row = np8 * 256;
-  // up to eight units (one warp each, about 200 registers a thread) per CTA
-  // and one CTA per SM; with one or two units, four or eight groups of rows
+  // up to eight units (one warp each, 218 registers a thread) per CTA and one CTA
+  // per SM; with one or two units, eight or four groups of rows.  Five or six
+  // units (17 to 24, 41 to 48 streams) leave the four schedulers one warp here
+  // and two there, so these take two groups too, in 10 or 12 warps of 168
+  // registers (17 words spilled): 0.1 to 0.2 s of 32 MS/s, 20
+  // streams, 4096 channels 0.733 -> 0.68 ms, 16384 channels 0.80 -> 0.77 (4x4
+  // register tiles 0.76); 48 streams, 1024 channels 1.18 -> 1.03 (1.78).  Past
+  // 64 streams a step of two rows is more than its 32 KB.
   p.nparts = (nunits + 7) / 8;
   p.upp = (nunits + p.nparts - 1) / p.nparts;
-  p.groups = p.upp == 1 ? 8 : p.upp == 2 ? 4 : p.upp <= 4 ? 2 : 1;
+  p.groups = p.upp == 1 ? 8 : p.upp == 2 ? 4 : p.upp <= 4 || (p.upp <= 6 && 2 * row <= 32768) ? 2 : 1;
   p.warps = p.upp * p.groups;
   p.R = std::max(p.groups, 32768 / row / p.groups * p.groups);
   p.smem = std::max((size_t)kRing * p.R * row, p.groups > 1 ? (size_t)p.groups / 2 * p.upp * 16384 : 0);
@@ -321,8 +328,9 @@ void launch_xcorr_f32(const float2 *spec, int nrows_total, int kpad, int nstream
   a.nbl = nbl;
   a.acc = acc;
   a.part = p.slots > 1 ? scratch : nullptr;
-  cudaFuncSetAttribute(xcorr_tile8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
-  xcorr_tile8_kernel<<<p.ctas, p.warps * 32, p.smem, st>>>(a);
+  auto kern = p.warps > 8 ? xcorr_tile8_kernel<384> : xcorr_tile8_kernel<256>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+  kern<<<p.ctas, p.warps * 32, p.smem, st>>>(a);
   if (a.part)
     tile8_reduce_kernel<<<dim3((K + 255) / 256, nbl), 256, 0, st>>>(scratch, blpart, p.nparts, p.nsteps, p.total, p.ctas,
                                                                     nbl, kpad, K, acc);

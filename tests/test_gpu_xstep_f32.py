@@ -42,7 +42,9 @@ def test_fp32_xstep_shapes(streams, rows, ref, pols):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("streams,rows,ref", [(35, 40, -1), (65, 12, -1), (72, 300, 1), (100, 9, -1), (128, 5, 2)])
+@pytest.mark.parametrize("streams,rows,ref", [(20, 600, -1), (35, 40, -1), (48, 300, -1), (65, 12, -1), (72, 300, 1),
+                                              (100, 9, -1), (128, 5, 2)])
 def test_fp32_xstep_wide(streams, rows, ref):
-    """Parts that leave warps without a unit, steps of a single row (from 65 streams), up to 128 streams."""
+    """Five and six units in two row groups, parts that leave warps without a
+    unit, steps of a single row (from 65 streams), up to 128 streams."""
     test_fp32_xstep_shapes(streams, rows, ref, 1)
