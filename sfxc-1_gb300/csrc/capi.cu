@@ -779,7 +779,7 @@ StreamDev last_stream(const sfxc_gpu_ctx *c, int stream) {
   return d;
 }
 
-// Node interval (the device search's answer) of the first block start of a
+// Node interval of the first block start of a
 // launch; the block kernel walks forward from it.
 int spline_lo_for(const StreamDev &d, const std::vector<double> &x) {
   const double v = (double)(d.start_ticks + (int64_t)d.block0 * kNd * d.tps - d.scan_begin) * (1.0 / 512000000.0);
@@ -1248,9 +1248,9 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
         const size_t xcap = c->xpart.cap;
         const int2 *units = c->units.as<int2>();
         const int nunits = (int)c->jt.units.size(), *blpart = c->blpart.as<int>();
-        q.kernel([=] {
-          launch_xcorr_f32(static_cast<float2 *>(specp), max_rows, kpad, N, npad, nrows, K, units, nunits, blmap, blpart,
-                           nbl, acc, xpart, xcap, xs);
+        q.op([=] {
+          return launch_xcorr_f32(static_cast<float2 *>(specp), max_rows, kpad, N, npad, nrows, K, units, nunits, blmap,
+                                  blpart, nbl, acc, xpart, xcap, xs);
         });
       }
       if (c->npc > 1) {  // the sub-integration into every phase centre

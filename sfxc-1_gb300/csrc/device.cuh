@@ -99,24 +99,13 @@ struct StreamDev {
 // --------------------------------------------------------------------------
 // FP64 Akima evaluation with the same operation order as the host (no FMA
 // contraction) so that integer delays agree bit for bit.
-__device__ __forceinline__ int spline_index(const double *x, int n, double v) {
-  int lo = 0, hi = n - 1;
-  while (hi > lo + 1) {
-    int i = (hi + lo) >> 1;
-    if (x[i] > v)
-      hi = i;
-    else
-      lo = i;
-  }
-  return lo;
-}
-// The interval spline_index finds for v, walking forward from lo, an
-// interval at or before it (spline_index is non-decreasing in v).
+// The node interval that holds v (the last node at or before it, at most the
+// last but one), walking forward from lo, an interval at or before it.
 __device__ __forceinline__ int spline_walk(const double *x, int n, double v, int lo) {
   while (lo < n - 2 && x[lo + 1] <= v) lo++;
   return lo;
 }
-// Evaluation in node interval i (as found by spline_index or spline_walk).
+// Evaluation in node interval i (as found by spline_walk).
 __device__ __forceinline__ double spline_eval_at(const double *sp, int n, int col, double v, int i) {
   const double *x = sp;
   const double *y = sp + n + col * 4 * n;
@@ -125,31 +114,6 @@ __device__ __forceinline__ double spline_eval_at(const double *sp, int n, int co
   double t = __dadd_rn(c[i], __dmul_rn(d[i], dx));
   t = __dadd_rn(b[i], __dmul_rn(dx, t));
   return __dadd_rn(y[i], __dmul_rn(dx, t));
-}
-__device__ __forceinline__ double spline_eval(const double *sp, int n, int col, double v) {
-  const double *x = sp;
-  const double *y = sp + n + col * 4 * n;
-  const double *b = y + n, *c = y + 2 * n, *d = y + 3 * n;
-  int i = spline_index(x, n, v);
-  double dx = __dsub_rn(v, x[i]);
-  double t = __dadd_rn(c[i], __dmul_rn(d[i], dx));
-  t = __dadd_rn(b[i], __dmul_rn(dx, t));
-  return __dadd_rn(y[i], __dmul_rn(dx, t));
-}
-__device__ __forceinline__ double time_diff_dev(int64_t a, int64_t b) {
-  return __ddiv_rn((double)(a - b), 512000000.0);
-}
-__device__ __forceinline__ double stream_delay(const StreamDev &s, int64_t t) {
-  double r = spline_eval(s.spline, s.spline_n, 0, time_diff_dev(t, s.scan_begin));
-  if (s.no_clock) return __dadd_rn(r, 0.0);
-  double drift = __dadd_rn(s.clock_offset, __dmul_rn(time_diff_dev(t, s.clock_epoch), s.clock_rate));
-  return __dadd_rn(r, drift);
-}
-__device__ __forceinline__ double stream_phase(const StreamDev &s, int64_t t) {
-  return spline_eval(s.spline, s.spline_n, 1, time_diff_dev(t, s.scan_begin));
-}
-__device__ __forceinline__ double stream_amplitude(const StreamDev &s, int64_t t) {
-  return spline_eval(s.spline, s.spline_n, 2, time_diff_dev(t, s.scan_begin));
 }
 
 // Named barrier `id` (1..15) over `count` threads (a multiple of 32) of the CTA.
@@ -195,11 +159,6 @@ __device__ __forceinline__ int find_segment(const StreamDev &s, int o) {
 // phase at channel 0, phase step per channel (rad), amplitude.
 struct UvShift {
   double phi, delta, amp, pad;
-};
-
-// Accumulator element written by the X kernels and read by normalisation.
-struct VisLayout {
-  int32_t nbl, kpad;  // baselines, padded channel count
 };
 
 // One output byte of channel extraction: spb = 8 / fan_out samples from the

@@ -42,14 +42,13 @@ struct TileArgs {
 };
 // the units of a job and the part of them each baseline's sums come from
 std::vector<int2> tile8_units(const std::vector<int> &blmap, int npad, int nstreams, std::vector<int> &blpart, int nbl);
-// Scratch it wants for its shares' partial sums (0: none); with less, each
-// CTA takes one whole column.
+// Scratch it needs for its shares' partial sums (0: none).
 size_t xcorr_f32_scratch_bytes(int nunits, int nstreams, int K, int nrows, int nbl, int kpad);
 // rows 0..nrows-1 of spec into acc.  Deterministic: every accumulator entry
 // has one writer, partial sums are added in a fixed order.
-void launch_xcorr_f32(const float2 *spec, int nrows_total, int kpad, int nstreams, int npad, int nrows, int K,
-                      const int2 *units, int nunits, const int *blmap, const int *blpart, int nbl, float2 *acc,
-                      float2 *scratch, size_t scratch_bytes, cudaStream_t st);
+cudaError_t launch_xcorr_f32(const float2 *spec, int nrows_total, int kpad, int nstreams, int npad, int nrows, int K,
+                             const int2 *units, int nunits, const int *blmap, const int *blpart, int nbl, float2 *acc,
+                             float2 *scratch, size_t scratch_bytes, cudaStream_t st);
 // FP32 X-step with pulsar binning (xcorr_f32_kernel): launch arguments and work split
 constexpr int kF32Stages = 4;         // cp.async ring depth
 constexpr int kF32StageBytes = 32768;  // rows x streams x 32 channels staged per step, at most

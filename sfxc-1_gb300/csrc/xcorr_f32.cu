@@ -297,16 +297,12 @@ size_t xcorr_f32_scratch_bytes(int nunits, int nstreams, int K, int nrows, int n
   return p.slots > 1 ? (size_t)p.slots * nbl * kpad * sizeof(float2) : 0;
 }
 
-void launch_xcorr_f32(const float2 *spec, int nrows_total, int kpad, int nstreams, int npad, int nrows, int K,
-                      const int2 *units, int nunits, const int *blmap, const int *blpart, int nbl, float2 *acc,
-                      float2 *scratch, size_t scratch_bytes, cudaStream_t st) {
-  if (nrows <= 0 || K <= 0 || nunits <= 0) return;
-  TilePlan p = tile_plan(nunits, nstreams, K, nrows);
-  if (p.slots > 1 && (!scratch || scratch_bytes < (size_t)p.slots * nbl * kpad * sizeof(float2))) {
-    // no room for partial sums: each share exactly one column
-    p.ctas = p.nct * p.nparts;
-    p.slots = 1;
-  }
+cudaError_t launch_xcorr_f32(const float2 *spec, int nrows_total, int kpad, int nstreams, int npad, int nrows, int K,
+                             const int2 *units, int nunits, const int *blmap, const int *blpart, int nbl, float2 *acc,
+                             float2 *scratch, size_t scratch_bytes, cudaStream_t st) {
+  if (nrows <= 0 || K <= 0 || nunits <= 0) return cudaSuccess;
+  const TilePlan p = tile_plan(nunits, nstreams, K, nrows);
+  if (p.slots > 1 && scratch_bytes < (size_t)p.slots * nbl * kpad * sizeof(float2)) return cudaErrorInvalidValue;
   TileArgs a;
   a.spec = spec;
   a.nrows_total = nrows_total;
@@ -334,6 +330,7 @@ void launch_xcorr_f32(const float2 *spec, int nrows_total, int kpad, int nstream
   if (a.part)
     tile8_reduce_kernel<<<dim3((K + 255) / 256, nbl), 256, 0, st>>>(scratch, blpart, p.nparts, p.nsteps, p.total, p.ctas,
                                                                     nbl, kpad, K, acc);
+  return cudaGetLastError();
 }
 
 }  // namespace sfxc
