@@ -558,8 +558,9 @@ void sfxc_gpu_batch_destroy(sfxc_gpu_batch *batch);
  * integration). */
 int sfxc_gpu_autotune(sfxc_gpu_ctx *ctx, int32_t trials);
 /* The plan cache: up to `capacity` entries of 5 int32 (kernel: 0 block stage,
- * 1 windowed FFT; two or three shape values; the chosen variant); returns the
- * number of entries. */
+ * 1 windowed FFT; three shape values -- streams, log2 of the blocks, 0, or FFT
+ * length, streams, log2 of the rows + 256 x stream slots of the tensor-core
+ * spectra layout; the chosen variant); returns the number of entries. */
 int sfxc_gpu_plan_cache(int32_t *out, int32_t capacity);
 
 /* Compute peaks of `device` for the rooflines (no counterpart in the

@@ -348,8 +348,10 @@ int ilog2c(int x) {
   return l;
 }
 std::array<int, 4> block_key(int nstreams, int max_blocks) { return {kKnobBlockStage, nstreams, ilog2c(max_blocks), 0}; }
-std::array<int, 4> window_key(int rot, int nstreams, int nrows) {
-  return {kKnobWindowFft, rot, nstreams, ilog2c(nrows)};
+// tc_slots: the spectra layout (0: FP32), whose kernels take different numbers of
+// streams and rows per CTA
+std::array<int, 4> window_key(int rot, int nstreams, int nrows, int tc_slots) {
+  return {kKnobWindowFft, rot, nstreams, ilog2c(nrows) + 256 * tc_slots};
 }
 int plan_get(const std::array<int, 4> &k) {
   std::lock_guard<std::mutex> lock(g_plan_mu);
@@ -1195,7 +1197,7 @@ void enqueue_integration(sfxc_gpu_ctx *c, int k = 0, bool require_push = true) {
       const float *win = t.window.as<float>();
       const float2 *twr = t.twrot.as<float2>();
       void *spec = c->spec.p;
-      const int ww = plan_get(window_key(rot, count, nrows));
+      const int ww = plan_get(window_key(rot, count, nrows, tc_slots));
       int *derr = device_error(c);
       q.kernel([=] {
         launch_window_fft(dchunk + N + first, count, 0, nrows, max_rows, win, twr, rot, nper, M, kpad, spec, tc_slots,
@@ -1699,7 +1701,7 @@ int sfxc_gpu_autotune(sfxc_gpu_ctx *c, int32_t trials) {
           best_v = v;
         }
       }
-      plan_set(window_key(rot, count, t.nrows), best_v);
+      plan_set(window_key(rot, count, t.nrows, t.tc_slots), best_v);
       tuned++;
     }
     cudaEventDestroy(e0);
