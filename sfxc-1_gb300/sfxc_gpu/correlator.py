@@ -60,7 +60,14 @@ def _collect(pieces, kind):
             C.memmove(*c)
     else:
         with ThreadPoolExecutor(max_workers=min(8, len(chunks), -(-total // _COPY_CHUNK))) as pool:
-            for f in [pool.submit(C.memmove, *c) for c in chunks]:
+            copies = []
+            try:
+                for c in chunks:
+                    copies.append(pool.submit(C.memmove, *c))
+            except RuntimeError:  # no (more) threads, as when the interpreter is shutting down
+                for c in chunks[len(copies):]:
+                    C.memmove(*c)
+            for f in copies:
                 f.result()
     return obj
 
