@@ -391,16 +391,36 @@ __global__ void __launch_bounds__(PackWin<LOGN, OUT_TC>::THREADS, 1)
   }
 }
 
+// Rows a group of threads takes in one run, with one CTA per SM, `groups` groups a
+// CTA and nsg groups of streams: the CTAs fill `waves` waves (the autotuner's
+// count), or by default two, or from 2048 points on one where that takes less time
+// counted in rows, the CTA's start (its tables, the first row's samples) being
+// about one.  Short runs of few streams gain by one wave (4 streams, 4096
+// channels, 976 rows, one wave of 7 against two of 4: tensor-core layout 0.84
+// of the time, FP32 0.86), long ones fill the SMs more evenly in two (32
+// streams, 4096 points, FP32 layout, 1952 rows: one wave 1.02); over 264 shapes
+// of 1 to 32 streams from 2048 points on, the rule takes 0.924 of two waves' time
+// in the mean and at most 1.015.
+int run_rows(int nsg, int nrows, int groups, int waves, bool long_start) {
+  auto rows = [&](int w) {
+    const int ctas = std::max(1, w * sm_count() / nsg);
+    return std::max(1, (nrows + ctas * groups - 1) / (ctas * groups));
+  };
+  auto time = [&](int r) {
+    const int grid = nsg * ((nrows + r * groups - 1) / (r * groups));
+    return (long long)((grid + sm_count() - 1) / sm_count()) * (r + 1);
+  };
+  if (waves > 0) return rows(waves);
+  return long_start && time(rows(1)) < time(rows(2)) ? rows(1) : rows(2);
+}
+
 template <int LOGN, int OUT_TC>
 void pack_launch(const StreamDev *d_streams, int nstreams, int row0, int nrows, int nrows_total, const float *window,
                  const float2 *tw_rot, int nper, int M, int kpad, void *spec, float tc_scale, int *err, cudaStream_t st,
                  int waves) {
   using W = PackWin<LOGN, OUT_TC>;
   const int nsg = (nstreams + W::NS - 1) / W::NS;
-  // one CTA per SM; runs of rows (one per group) so that the CTAs fill two
-  // waves by default (the autotuner may pick another count per shape)
-  const int ctas = std::max(1, (waves > 0 ? waves : 2) * sm_count() / nsg);
-  const int rows_per_group = std::max(1, (nrows + ctas * W::GROUPS - 1) / (ctas * W::GROUPS));
+  const int rows_per_group = run_rows(nsg, nrows, W::GROUPS, waves, W::BULK);
   const unsigned grid = (unsigned)(nsg * ((nrows + rows_per_group * W::GROUPS - 1) / (rows_per_group * W::GROUPS)));
   auto kern = window_pack_kernel<LOGN, OUT_TC>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)W::SMEM);
@@ -605,8 +625,7 @@ template <int OUT_TC>
 void long_launch(const StreamDev *d_streams, int nstreams, int row0, int nrows, int nrows_total, const float *window,
                  const float2 *tw_rot, int nper, int M, int kpad, void *spec, float tc_scale, int *err, cudaStream_t st,
                  int waves) {
-  const int ctas = std::max(1, (waves > 0 ? waves : 2) * sm_count() / nstreams);
-  const int rows_per_group = std::max(1, (nrows + ctas - 1) / ctas);
+  const int rows_per_group = run_rows(nstreams, nrows, 1, waves, true);
   const unsigned grid = (unsigned)(nstreams * ((nrows + rows_per_group - 1) / rows_per_group));
   auto kern = window_long_kernel<OUT_TC>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LongWin::SMEM);
