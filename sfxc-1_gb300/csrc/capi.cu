@@ -1630,10 +1630,16 @@ int sfxc_gpu_copy_unpacked(sfxc_gpu_ctx *c, int32_t stream, float *out, size_t n
     const size_t need = (size_t)s.n_blocks * c->Nd;
     if (n < need) throw Error(SFXC_GPU_EINVAL, "output buffer too small");
     StreamDev d = last_stream(c, stream);
-    DevBuf sd, dout;
+    d.block0 = 0;
+    d.n_blocks = s.n_blocks;
+    d.spline_lo = spline_lo_for(d, s.sp.x);
+    DevBuf sd, dout, bp;
     dout.ensure(need * sizeof(float));
+    bp.ensure((size_t)s.n_blocks * sizeof(BlockPar));
+    d.bpar = bp.as<BlockPar>();
     upload(sd, &d, sizeof(StreamDev), c->st);
-    launch_unpack(sd.as<StreamDev>(), 1, s.n_blocks, dout.as<float>(), c->st);
+    launch_block_params(sd.as<StreamDev>(), 1, s.n_blocks, c->st);
+    launch_unpack(sd.as<StreamDev>(), s.n_blocks, dout.as<float>(), c->st);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(out, dout.p, need * sizeof(float), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));

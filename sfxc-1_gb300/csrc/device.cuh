@@ -131,17 +131,6 @@ __device__ __forceinline__ float code_value2(uint32_t c) {
   return __int_as_float((int)__byte_perm(0x4040C0C0u, 0xE00000E0u, c * 0x1100u + 0x0455u));
 }
 
-// Unpacked sample `o` (index within the integration) through the plan;
-// `si` is a segment cursor that only moves forward for increasing `o`.
-__device__ __forceinline__ float gather_sample(const StreamDev &s, int o, int &si) {
-  while (si + 1 < s.nsegs && s.segs[si].out0 + s.segs[si].n <= o) si++;
-  const DevSegment sg = s.segs[si];
-  if (sg.src_bit < 0 || o < sg.out0 || o >= sg.out0 + sg.n) return 0.0f;
-  const int64_t bit = sg.src_bit + (int64_t)(o - sg.out0) * s.bits;
-  const int code = (__ldg(s.src + (bit >> 3)) >> (bit & 7)) & ((1 << s.bits) - 1);
-  // Bit2float_worker lookup tables (sfxc/src/bit2float_worker.cc:4-10)
-  return s.bits == 2 ? (code == 0 ? -7.f : code == 1 ? -2.f : code == 2 ? 2.f : 7.f) : (code ? 5.f : -5.f);
-}
 // First segment whose range can contain sample o (binary search on out0).
 __device__ __forceinline__ int find_segment(const StreamDev &s, int o) {
   int lo = 0, hi = s.nsegs - 1;

@@ -188,6 +188,23 @@ struct Rotor {
   }
 };
 
+// Unpacked samples of one stream's blocks (inspection of the Bit2float_worker
+// output), by the block stage's own unpacking: a half warp per pair of blocks.
+__global__ void __launch_bounds__(kThreads) unpack_kernel(const StreamDev *__restrict__ stream, float *__restrict__ out) {
+  __shared__ __align__(16) uint32_t words[kThreads / 16][64];
+  const StreamDev &s = *stream;
+  const int t = threadIdx.x & 15, grp = threadIdx.x >> 4, bl = (blockIdx.x * (kThreads / 16) + grp) * 2;
+  if ((bl & ~3) >= s.n_blocks) return;  // whole warps (four blocks each)
+  float x0[16], x1[16];
+  unpack_pair(s.bits == 2, fetch_pair(s, s.bpar + bl, bl, t), t, words[grp], x0, x1);
+#pragma unroll
+  for (int r = 0; r < 16; r++) {
+    float *const o = out + (int64_t)bl * kNd + t + 16 * r;
+    if (bl < s.n_blocks) o[0] = x0[r];
+    if (bl + 1 < s.n_blocks) o[kNd] = x1[r];
+  }
+}
+
 // CTAs of 64 blocks a round, rounds strided over the stream's blocks.
 __global__ void __launch_bounds__(kThreads, 2) fstep_block_kernel(const StreamDev *__restrict__ streams,
                                                                  const float2 *__restrict__ tw) {
@@ -362,6 +379,11 @@ __global__ void __launch_bounds__(kThreads, 2) fstep_block_kernel(const StreamDe
 }
 
 }  // namespace
+
+void launch_unpack(const StreamDev *d_stream, int n_blocks, float *out, cudaStream_t st) {
+  constexpr int per_cta = kThreads / 8;
+  unpack_kernel<<<(n_blocks + per_cta - 1) / per_cta, kThreads, 0, st>>>(d_stream, out);
+}
 
 void launch_fstep(const StreamDev *d_streams, int nstreams, int max_blocks, const float2 *tw256, cudaStream_t st,
                   int ctas_per_sm) {

@@ -112,15 +112,6 @@ __device__ __forceinline__ void block_params_one(const StreamDev &s, int bl, int
   s.bpar[bl] = bp;
 }
 
-// Unpacked samples only (inspection of the Bit2float_worker output).
-__global__ void unpack_kernel(const StreamDev *__restrict__ streams, float *__restrict__ out) {
-  const StreamDev &s = streams[blockIdx.y];
-  const int o0 = (s.block0 + blockIdx.x) * kNd;
-  if ((int)blockIdx.x >= s.n_blocks) return;
-  int si = find_segment(s, o0 + threadIdx.x);
-  out[(int64_t)blockIdx.x * kNd + threadIdx.x] = gather_sample(s, o0 + threadIdx.x, si);
-}
-
 // Channel extraction: output byte `ob` of subband s packs spb = 8/fan_out
 // samples (extract_byte); sample j reads word ob*spb+j.
 __global__ void extract_kernel(const uint8_t *__restrict__ in, int64_t nout, int N, int bits, int fan_out,
@@ -725,10 +716,6 @@ void launch_fstep_block(const StreamDev *d_streams, int nstreams, int max_blocks
                         cudaStream_t st) {
   launch_block_params(d_streams, nstreams, max_blocks, st);
   launch_fstep(d_streams, nstreams, max_blocks, tw256, st, 0);
-}
-
-void launch_unpack(const StreamDev *d_streams, int nstreams, int max_blocks, float *out, cudaStream_t st) {
-  unpack_kernel<<<dim3(max_blocks, nstreams), kNd, 0, st>>>(d_streams, out);
 }
 
 void launch_extract(const uint8_t *in, int64_t nout, int N, int bits, int nsub, int fan_out, const int *tracks,

@@ -19,7 +19,8 @@ void launch_block_params(const StreamDev *d_streams, int nstreams, int max_block
 // ctas_per_sm: grid of the block stage, CTAs per SM over all streams (0: the default, 10)
 void launch_fstep(const StreamDev *d_streams, int nstreams, int max_blocks, const float2 *tw256, cudaStream_t st,
                   int ctas_per_sm = 0);
-void launch_unpack(const StreamDev *d_streams, int nstreams, int max_blocks, float *out, cudaStream_t st);
+// samples of one stream's blocks as the block stage unpacks them, from its records (launch_block_params)
+void launch_unpack(const StreamDev *d_stream, int n_blocks, float *out, cudaStream_t st);
 void launch_extract(const uint8_t *in, int64_t nout, int N, int bits, int nsub, int fan_out, const int *tracks,
                     uint8_t *out, cudaStream_t st);
 // tc_slots: slots per (row, channel) of the TC layout (32 or 64); 0 writes the FP32 layout

@@ -48,3 +48,20 @@ def test_block_stage_unpacking(bits, block_bytes, rows, invalid):
     assert h0 == h1
     a, b = np.array(v0).astype(np.complex128), np.array(v1).astype(np.complex128)
     assert np.linalg.norm(a - b) < 2e-6 * np.linalg.norm(b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bits", [1, 2])
+@pytest.mark.parametrize("block_bytes,rows,invalid", [(2000, 9, []), (40, 34, [(7, 9)]), (2000, 131, [(100, 700), (900, 1)])])
+def test_unpacked_samples(bits, block_bytes, rows, invalid):
+    """The samples themselves, bit for bit: the inspection call runs the block stage's own unpacking."""
+    j = make_job(bits, block_bytes, rows, invalid)
+    want = jobs.correlate(j, dump=True, impl="oracle")["unpacked"]
+    node = correlator.CorrelatorNode(0, lib.X_FP32)
+    try:
+        node.correlate(j)
+        for k in range(2):
+            assert np.array_equal(node.unpacked(k, want[(0, k)].size), want[(0, k)])
+            assert invalid == [] or k == 1 or (want[(0, k)] == 0).any()
+    finally:
+        node.close()
