@@ -393,15 +393,13 @@ __global__ void __launch_bounds__(PackWin<LOGN, OUT_TC>::THREADS, 1)
 
 // Rows a group of threads takes in one run, with one CTA per SM, `groups` groups a
 // CTA and nsg groups of streams: the CTAs fill `waves` waves (the autotuner's
-// count), or by default two, or from 2048 points on one where that takes less time
-// counted in rows, the CTA's start (its tables, the first row's samples) being
-// about one.  Short runs of few streams gain by one wave (4 streams, 4096
-// channels, 976 rows, one wave of 7 against two of 4: tensor-core layout 0.84
-// of the time, FP32 0.86), long ones fill the SMs more evenly in two (32
-// streams, 4096 points, FP32 layout, 1952 rows: one wave 1.02); over 264 shapes
-// of 1 to 32 streams from 2048 points on, the rule takes 0.924 of two waves' time
-// in the mean and at most 1.015.
-int run_rows(int nsg, int nrows, int groups, int waves, bool long_start) {
+// count), or by default two, or one where that takes less than `percent` of the
+// time, counted in rows with the CTA's start (its tables, the first row's samples)
+// as one.  Short runs of few streams gain by one wave (4 streams, 4096 channels,
+// 976 rows, one wave of 7 rows a run against two of 4: 0.84 of the time in the
+// tensor-core layout, 0.86 in FP32); where the counts are close, two waves even
+// out the SMs (32 streams, 8192 points, FP32, 1952 rows: one wave 1.07).
+int run_rows(int nsg, int nrows, int groups, int waves, int percent) {
   auto rows = [&](int w) {
     const int ctas = std::max(1, w * sm_count() / nsg);
     return std::max(1, (nrows + ctas * groups - 1) / (ctas * groups));
@@ -411,8 +409,13 @@ int run_rows(int nsg, int nrows, int groups, int waves, bool long_start) {
     return (long long)((grid + sm_count() - 1) / sm_count()) * (r + 1);
   };
   if (waves > 0) return rows(waves);
-  return long_start && time(rows(1)) < time(rows(2)) ? rows(1) : rows(2);
+  return time(rows(1)) * 100 < time(rows(2)) * percent ? rows(1) : rows(2);
 }
+// From 2048 points on: over 456 shapes (1 to 32 streams, 16 to 125 ms of 32 and 64
+// MS/s) 0.932 of two waves' time in the mean, at most 1.04.  The one-stream
+// kernel's 8-byte pieces in the tensor-core layout lose up to 5 % in one wave where
+// the counts are within a twentieth (24 streams, 488 rows).
+constexpr int kOneWave = 97, kOneWaveLongTc = 94;
 
 template <int LOGN, int OUT_TC>
 void pack_launch(const StreamDev *d_streams, int nstreams, int row0, int nrows, int nrows_total, const float *window,
@@ -420,7 +423,7 @@ void pack_launch(const StreamDev *d_streams, int nstreams, int row0, int nrows, 
                  int waves) {
   using W = PackWin<LOGN, OUT_TC>;
   const int nsg = (nstreams + W::NS - 1) / W::NS;
-  const int rows_per_group = run_rows(nsg, nrows, W::GROUPS, waves, W::BULK);
+  const int rows_per_group = run_rows(nsg, nrows, W::GROUPS, waves, W::BULK ? kOneWave : 0);
   const unsigned grid = (unsigned)(nsg * ((nrows + rows_per_group * W::GROUPS - 1) / (rows_per_group * W::GROUPS)));
   auto kern = window_pack_kernel<LOGN, OUT_TC>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)W::SMEM);
@@ -625,7 +628,7 @@ template <int OUT_TC>
 void long_launch(const StreamDev *d_streams, int nstreams, int row0, int nrows, int nrows_total, const float *window,
                  const float2 *tw_rot, int nper, int M, int kpad, void *spec, float tc_scale, int *err, cudaStream_t st,
                  int waves) {
-  const int rows_per_group = run_rows(nstreams, nrows, 1, waves, true);
+  const int rows_per_group = run_rows(nstreams, nrows, 1, waves, OUT_TC ? kOneWaveLongTc : kOneWave);
   const unsigned grid = (unsigned)(nstreams * ((nrows + rows_per_group - 1) / rows_per_group));
   auto kern = window_long_kernel<OUT_TC>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LongWin::SMEM);
