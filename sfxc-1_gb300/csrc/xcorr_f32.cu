@@ -26,12 +26,16 @@ namespace {
 // Bounds: FP32 multiply-adds with three register operands, which run at 26 of
 // 38 T lane operations/s here; three quarters of the instructions are such,
 // the pipe is 55 % busy.  32 streams, 4096 channels, 62.5 ms of 64 MS/s:
-// 0.42 ms where 4x4 tiles in registers took 0.76 (22 % against 45 % of the
+// 0.43 ms where 4x4 tiles in registers took 0.76 (22 % against 45 % of the
 // shared-memory bandwidth); whole jobs beside their F-step: 32 streams, 1 s,
-// 22.6 -> 18.3 ms, 16 streams, 0.5 s, 5.5 -> 4.2 ms.  Two to five small CTAs
+// 22.6 -> 18.6 ms, 16 streams, 0.5 s, 5.5 -> 4.25 ms.  Two to five small CTAs
 // per SM instead of row groups took 5.4 ms on the latter (single-row steps).
 constexpr int kRing = 4;
-constexpr int kRun = 256;  // rows a thread sums in registers at most: longer sums would lose more to rounding
+// Rows a thread sums in registers at most; longer sums lose more to rounding, and
+// shorter ones cost more flushes.  33 streams, 1952 rows, autocorrelations against
+// FP64: 9.4e-8 (1.37e-7 with 256 rows; 1.19e-7 for blocks of about 200 rows of the
+// 4x4 tiles), in the mean over 62 shapes 2.5 % of the X-step and 1.2 % of a job.
+constexpr int kRun = 128;
 
 // first step of CTA i's share
 __device__ __host__ __forceinline__ long long share_begin(long long total, int ctas, int i) { return total * i / ctas; }

@@ -48,3 +48,30 @@ def test_fp32_xstep_wide(streams, rows, ref):
     """Five and six units in two row groups, parts that leave warps without a
     unit, steps of a single row (from 65 streams), up to 128 streams."""
     test_fp32_xstep_shapes(streams, rows, ref, 1)
+
+
+@pytest.mark.gpu
+def test_fp32_xstep_sum_rounding():
+    """Rounding of long sums: autocorrelations of 1952 rows against FP64, root
+    mean square over streams and channels.
+
+    Two roundings a row of a partial sum that grows evenly, each 2.4e-8 of it in
+    the root mean square: sqrt(2 x 128 / 3) of them in a run of 128 rows, averaged
+    over 15 runs, 5.8e-8; the 15 runs' sums, sqrt(15 / 3) of them, 5.4e-8;
+    accumulator and normalisation 4e-8; the transforms' fixed factors up to 7e-8:
+    1.2e-7 in quadrature.  (Runs of 256 rows: 1.2e-7 by themselves.)"""
+    rate, nchan = 32_000_000, 1024
+    sc = scenario.Scenario(stations=scenario.cubic_stations(33, seed=2, max_delay=1e-4, max_rate=1e-6), sample_rate=rate,
+                           bandwidth=rate // 2, nchan=nchan, integration_us=62500, n_integrations=1, lead_us=1000, seed=11,
+                           block_bytes=2000)
+    j = scenario.build_job_bulk(sc)
+    jj = dict(j, protocols=[[bytes(p) for p in s] for s in j["protocols"]])
+    want = jobs.correlate(jj, impl="oracle", precision=64)["cor"]
+    node = correlator.CorrelatorNode(0, lib.X_FP32)
+    try:
+        got, _ = node.correlate(j)
+    finally:
+        node.close()
+    a, b = (np.array(correlator.split_output(x, nchan)[1])[:33, 1:-1].real.astype(np.float64) for x in (got, want))
+    rms = np.sqrt((((a - b) / b)**2).mean())
+    assert rms < 1.2e-7
