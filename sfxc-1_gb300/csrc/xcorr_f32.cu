@@ -19,9 +19,12 @@ namespace {
 // they multiply).  A diagonal unit takes two diagonal tiles a and b, the upper
 // triangle of a above its diagonal, that of b below, and both tiles'
 // autocorrelations, which are real, on it.  Where the units are few, groups of
-// warps take every G-th row and add their tiles up in shared memory.  A share's
-// sums of a column go to a slot of the partial sums, added later in order, so
-// results do not depend on timing.
+// warps each take a stretch of consecutive rows and add their tiles up in shared
+// memory (every G-th row instead lost the cancellation of products that turn by
+// 1/G from row to row, as a tone's do at some fringe rates: errors of 5e-8 of the
+// terms' sum where consecutive rows lose 1e-9).  A share's sums of a column go to
+// a slot of the partial sums, added later in order, so results do not depend on
+// timing.
 //
 // Bounds: FP32 multiply-adds with three register operands, which run at 26 of
 // 38 T lane operations/s here; three quarters of the instructions are such,
@@ -72,12 +75,16 @@ __device__ __forceinline__ void tile_row(float2 (&v)[8][8], const float2 *xa, co
     }
 }
 
-template <int THREADS>
+// GROUPS: row groups, 0 for one (with the count a constant 1 the compiler's code
+// for that case was 3 to 6 % slower)
+template <int THREADS, int GROUPS>
 __global__ void __launch_bounds__(THREADS, 1) xcorr_tile8_kernel(const __grid_constant__ TileArgs a) {
   extern __shared__ __align__(16) float2 xs[];  // kRing x [R rows][np8 streams][32 channels]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, G = a.groups;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int G = GROUPS > 0 ? GROUPS : a.groups;
   const int wu = warp % a.units_per_part, wg = warp / a.units_per_part;  // unit of the part, row group
   const int stage = a.R * a.np8 * 32, rstride = a.np8 * 32;
+  const int gstep = a.R / G;
   const int run = max(1, kRun * G / a.R);
   const long long total = (long long)a.nct * a.nparts * a.nsteps;
   const long long w0 = share_begin(total, gridDim.x, blockIdx.x), w1 = share_begin(total, gridDim.x, blockIdx.x + 1);
@@ -97,20 +104,38 @@ __global__ void __launch_bounds__(THREADS, 1) xcorr_tile8_kernel(const __grid_co
     // channel kk + 1 may be K, which lies inside the padded row (kpad >= K + 3)
     const bool kok = ct * 32 + cc < a.K;
     const float2 *const src0 = a.spec + (int64_t)st0 * sstride + ct * 32 + cc;
+    // a step stages R / G rows of each row group, from the group's stretch of ns R / G;
+    // row rr of group g in slot rr G + g
+    const int gspan = ns * gstep;
+    const int64_t gstride = gspan * (int64_t)a.kpad;
     auto issue = [&](int step) {
       if (step < ns) {
-        const int row0 = (s0 + step) * a.R;
+        const int row0 = s0 * a.R + step * gstep;
         uint32_t d0 = ring0 + (uint32_t)((step % kRing) * stage) * 8u;
         const float2 *p0 = src0 + (int64_t)row0 * a.kpad;
         for (int st = st0; st < a.np8; st += dst_st) {
           const bool ok = kok && st < a.nstreams;
           const float2 *p = p0;
           uint32_t d = d0;
-          for (int rr = 0; rr < a.R; rr++) {
-            const bool in = ok && row0 + rr < a.nrows;
-            tc::cp_async16(d, in ? p : a.spec, in ? 16 : 0);
-            p += a.kpad;
-            d += rstride * 8;
+          if constexpr (GROUPS > 0) {
+            for (int rr = 0; rr < gstep; rr++) {
+              const float2 *q = p;
+#pragma unroll
+              for (int g = 0; g < GROUPS; g++) {
+                const bool in = ok && row0 + rr + g * gspan < a.nrows;
+                tc::cp_async16(d, in ? q : a.spec, in ? 16 : 0);
+                q += gstride;
+                d += rstride * 8;
+              }
+              p += a.kpad;
+            }
+          } else {
+            for (int rr = 0; rr < a.R; rr++) {
+              const bool in = ok && row0 + rr < a.nrows;
+              tc::cp_async16(d, in ? p : a.spec, in ? 16 : 0);
+              p += a.kpad;
+              d += rstride * 8;
+            }
           }
           p0 += dst_st * sstride;
           d0 += dst_st * 256;
@@ -234,14 +259,14 @@ struct TilePlan {
 TilePlan tile_plan(int nunits, int nstreams, int K, int nrows) {
   TilePlan p{};
   const int np8 = (nstreams + 7) / 8 * 8, row = np8 * 256;
-  // up to eight units (one warp each, 218 registers a thread) per CTA and one CTA
+  // up to eight units (one warp each, 220 registers a thread) per CTA and one CTA
   // per SM; with one or two units, eight or four groups of rows.  Five or six
   // units (17 to 24, 41 to 48 streams) leave the four schedulers one warp here
   // and two there, so these take two groups too, in 10 or 12 warps of 168
-  // registers (17 words spilled): 0.1 to 0.2 s of 32 MS/s, 20
-  // streams, 4096 channels 0.733 -> 0.68 ms, 16384 channels 0.80 -> 0.77 (4x4
-  // register tiles 0.76); 48 streams, 1024 channels 1.18 -> 1.03 (1.78).  Past
-  // 64 streams a step of two rows is more than its 32 KB.
+  // registers (21 words spilled): 20 streams, 4096 channels, 0.2 s of 32 MS/s 0.764
+  // -> 0.727 ms, 16384 channels 0.817 -> 0.795 (4x4 register tiles 0.764); 48 streams,
+  // 1024 channels, 83 ms 1.18 -> 1.07 (1.78).  Past 64 streams a step of two rows is
+  // more than its 32 KB.
   p.nparts = (nunits + 7) / 8;
   p.upp = (nunits + p.nparts - 1) / p.nparts;
   p.groups = p.upp == 1 ? 8 : p.upp == 2 ? 4 : p.upp <= 4 || (p.upp <= 6 && 2 * row <= 32768) ? 2 : 1;
@@ -328,7 +353,11 @@ cudaError_t launch_xcorr_f32(const float2 *spec, int nrows_total, int kpad, int 
   a.nbl = nbl;
   a.acc = acc;
   a.part = p.slots > 1 ? scratch : nullptr;
-  auto kern = p.warps > 8 ? xcorr_tile8_kernel<384> : xcorr_tile8_kernel<256>;
+  auto kern = p.warps > 8     ? xcorr_tile8_kernel<384, 2>
+              : p.groups == 1 ? xcorr_tile8_kernel<256, 0>
+              : p.groups == 2 ? xcorr_tile8_kernel<256, 2>
+              : p.groups == 4 ? xcorr_tile8_kernel<256, 4>
+                              : xcorr_tile8_kernel<256, 8>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
   kern<<<p.ctas, p.warps * 32, p.smem, st>>>(a);
   if (a.part)

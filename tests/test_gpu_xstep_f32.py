@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 from oracle import jobs
-from sfxc_gpu import correlator, lib, scenario
+from sfxc_gpu import correlator, lib, scenario, synth
 
 
 def make_job(streams, rows, ref=-1, pols=1, seed=7):
@@ -75,3 +75,49 @@ def test_fp32_xstep_sum_rounding():
     a, b = (np.array(correlator.split_output(x, nchan)[1])[:33, 1:-1].real.astype(np.float64) for x in (got, want))
     rms = np.sqrt((((a - b) / b)**2).mean())
     assert rms < 1.2e-7
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("streams,period", [(2, 8), (2, 3), (7, 4), (16, 4), (20, 2), (24, 5), (34, 2)])
+def test_fp32_xstep_turning_products(streams, period):
+    """A tone in every station, half of them at a fringe rate that turns its
+    products with the others by 1 / period from row to row: they cancel, and the
+    rounding of their sum has to be that of consecutive rows, whose partial sums
+    stay at a few terms, whatever the work split.
+
+    Relative to the sum of the terms' moduli: the transforms' 2e-7 a row, which
+    differs from row to row, over 1950 rows 5e-9; two roundings a row of sums of
+    up to period / pi terms, below 2e-9; 2e-8 is allowed.  (Sums over every
+    period-th row grow to all their terms: 5e-8.)"""
+    rate, nchan, rows, sky, tone = 32_000_000, 256, 1953, 1_600_000_000, 3_968_750
+    r = rate / nchan / period / (sky + tone)  # seconds a second
+    st = [scenario.Station("S%d" % k, k, synth.DelayPoly(coeffs=(0.0, r if k % 2 else 0.0), t0=36000.0))
+          for k in range(streams)]
+    sc = scenario.Scenario(stations=st, sample_rate=rate, bandwidth=rate // 2, nchan=nchan, channel_freq=sky,
+                           integration_us=rows * nchan * 1_000_000 // rate, n_integrations=1, lead_us=1000, seed=1,
+                           block_bytes=2000)
+
+    def codes(k, nbytes):
+        n = 4 * nbytes
+        x = np.cos(2 * np.pi * tone / rate * np.arange(n)) + np.random.Generator(np.random.PCG64(k)).normal(size=n)
+        return synth.pack_codes(synth.quantise(x, 2), 2)
+
+    j = scenario.build_job_bulk(sc, codes=codes)
+    jj = dict(j, protocols=[[bytes(p) for p in s] for s in j["protocols"]])
+    want = jobs.correlate(jj, impl="oracle", precision=64)["cor"]
+    node = correlator.CorrelatorNode(0, lib.X_FP32)
+    try:
+        got, _ = node.correlate(j)
+    finally:
+        node.close()
+    a, b = (np.array(correlator.split_output(x, nchan)[1]).astype(np.complex128) for x in (got, want))
+    ch = round(tone / (rate / 2 / nchan))
+    assert np.argmax(b[0].real) in (ch - 1, ch, ch + 1)
+    pairs = [(p, q) for p in range(streams) for q in range(p + 1, streams)]
+    worst = 0.0
+    for v, w, (p, q) in zip(a[streams:], b[streams:], pairs):
+        if (p + q) % 2:
+            moduli = np.sqrt(b[p].real * b[q].real)
+            assert abs(w[ch]) < 0.05 * moduli[ch]  # the terms cancel
+            worst = max(worst, abs(v[ch] - w[ch]) / moduli[ch])
+    assert worst < 2e-8, worst
