@@ -21,7 +21,7 @@ namespace {
 // upper half zero, inverse 256-point transform (as conj(FFT(conj Y))), fringe
 // rotation of the real part.
 //
-// Bounds: 51 instructions per sample at 0.47 issued per cycle and scheduler
+// Bounds: 49 instructions per sample at 0.47 issued per cycle and scheduler
 // (16 warps per SM: a packed transform takes 64 registers), fetched as mostly
 // straight code by warps out of step with each other (a fifth of the stalls;
 // both inverses unrolled 3.46 ms, CTA-wide barriers 3.0 to 3.4), and 54 % of

@@ -31,7 +31,7 @@ namespace {
 // 0.78 ms against one group of threads per stream.  16384 points:
 // window_long_kernel.
 //
-// What bounds it: 40.7 instructions per point (73.5 with scalar FP32 and the
+// What bounds it: 42 instructions per point (73.5 with scalar FP32 and the
 // split through shared memory) and 59 bytes of shared-memory and L1 traffic
 // per point, by warps few enough (8 to 16 per SM, the transforms fill the
 // registers and 213 KB of shared memory) that latency counts.  Measured at 32
@@ -443,7 +443,7 @@ void pack_launch(const StreamDev *d_streams, int nstreams, int row0, int nrows, 
 // sector costs the L2 as much as a whole one); without them the chain of five
 // passes of 16 warps in step.  24 streams, 0.5 s of 64 MS/s: tensor-core layout
 // 5.53 -> 5.18 ms (5.49 with the whole window loaded after the samples have
-// landed), FP32 layout 3.55 -> 3.63 ms, against one scalar transform of 1024
+// landed), FP32 layout 3.55 -> 3.60 ms, against one scalar transform of 1024
 // threads.
 constexpr int kLongN = 16384;
 struct LongWin {
