@@ -318,7 +318,7 @@ def roofline(cfg, per_kernel, total, steps, peaks, x_mode, nbl_per_stream):
     # ncu measured for the tensor-core path's kernels on the one-subband,
     # 4096-channel case; a launch covers one sub-integration chunk of one
     # subband job, so the per-launch traffic scales with the samples it covers
-    measured = {"window_fft_ms": 11.87, "xstep_ms": 8.18, "unpack_fringe_ms": 4.27}
+    measured = {"window_fft_ms": 12.01, "xstep_ms": 8.18, "unpack_fringe_ms": 4.23}
     traffic = None
     if x_mode == "tc" and M == 4096 and k in measured and not cfg["pulsar"]:
         launches = cfg["subbands"] * -(-cfg["integration_us"] // 125000)
